@@ -346,6 +346,11 @@ __device__ __forceinline__ int sliver_mask(const ForceParams& P, float px, float
     return (px >= P.g.b_nx ? 1 : 0) | (py >= P.g.b_nx ? 2 : 0) | (D == 3 && pz >= P.g.b_nx ? 4 : 0);
 }
 
+// Grid row of cell c: c / nx.
+__device__ __forceinline__ int grid_row(uint32_t c, const ForceParams& P) {
+    return (int)(__umulhi(c, P.row_mul) >> P.row_shift);
+}
+
 template <int D>
 struct TileRows {
     static constexpr int R = D == 3 ? 9 : 3;
@@ -355,22 +360,32 @@ struct TileRows {
 // the target uses x - 1 (y - 1, z - 1) against it, because the candidate is
 // the periodic image above the box of a cell near coordinate 0.
 constexpr int kShiftX = 1 << 16, kShiftY = 1 << 17, kShiftZ = 1 << 18;
-// Staging only (never in a staged word): the cell's image lies below the box
-// in x or y and its candidates are shifted down by 1 as they are copied.
-constexpr int kNegX = 1 << 20, kNegY = 1 << 21;
-// Average staged candidates per cell from which a 2D block copies its cells
-// one warp per cell instead of one owner thread per cell.
-constexpr int kDenseCell = 16;
+// A staged cell's image shifts (TileSmem::image): it lies above the box in x,
+// y or z (its candidates are flagged kShift*), or below it (its candidates
+// are moved down by 1 as they are copied).
+constexpr int kUpX = 1, kUpY = 2, kUpZ = 4, kDownX = 8, kDownY = 16, kDownZ = 32;
+// Average staged candidates per cell from which a cell is copied by a whole
+// warp, and from which by 8 lanes (fewer: by 4): about one trip of the
+// group per cell with half of its lanes or more at work.
+constexpr int kDenseCell = 16, kSparseCell = 4;
 
-__device__ __forceinline__ int wrap_index(int c, int n) { return c < 0 ? c + n : (c >= n ? c - n : c); }
+// Asynchronous 16-byte copy from global to shared memory, and the wait for
+// this thread's copies.
+__device__ __forceinline__ void copy16_async(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// A staged candidate: coordinates of an image below the box moved down by
-// one, target-shift flags (images above the box) in the type word.
+// A staged candidate of an image cell: coordinates of an image below the box
+// moved down by one (exact: they are >= 0.5), target-shift flags of an image
+// above it in the type word.
 template <int D>
-__device__ __forceinline__ float4 shift_candidate(float4 q, float sx, float sy, float sz, int flags) {
-    q.x -= sx;
-    q.y -= sy;
-    if (D == 3) q.z -= sz;
+__device__ __forceinline__ float4 shift_candidate(float4 q, int image) {
+    q.x -= (image & kDownX) ? 1.f : 0.f;
+    q.y -= (image & kDownY) ? 1.f : 0.f;
+    if (D == 3) q.z -= (image & kDownZ) ? 1.f : 0.f;
+    const int flags = (image & (kUpX | kUpY | kUpZ)) * kShiftX;
     if constexpr (D == 2)
         q.z = __int_as_float(__float_as_int(q.z) | flags);
     else

@@ -50,6 +50,14 @@ void fill_force_params(const plg_settings& s, int nx, int64_t ncells, int ntypes
     p.wrap = s.wrap ? 1 : 0;
     p.ntypes = ntypes;
     p.slmask_ok = nx >= 4 ? 1 : 0;
+    // Division by nx as a multiplication (grid_row): with 2^(l-1) < nx <= 2^l
+    // and m = floor(2^(31+l) / nx) + 1, c m / 2^(31+l) exceeds c / nx by less
+    // than c / 2^31 / nx, so its floor is exact for c < 2^31 (nx >= 2; the
+    // tiled kernel runs for nx >= 3).
+    int l = 1;
+    while (((int64_t)1 << l) < nx) ++l;
+    p.row_mul = nx < 2 ? 0u : (uint32_t)(((uint64_t)1 << (31 + l)) / (uint64_t)nx + 1);
+    p.row_shift = l - 1;
     const double r2 = s.rmax * s.rmax;
     const double lo_d = r2 * (1.0 - kBandRel), hi_d = r2 * (1.0 + kBandRel);
     float lo = (float)lo_d, hi = (float)hi_d;
