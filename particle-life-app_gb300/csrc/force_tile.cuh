@@ -22,9 +22,10 @@
 // columns are staged in chunks (which may span segments), halved until they
 // fit, and a single window that still does not fit (a very dense region) is
 // read from global memory in the same candidate order (direct_stencil),
-// giving the same bits.  The
-// candidate loop is branch-free FP32.  A target that meets a candidate
-// needing the FP64 decision is deferred: its warp recomputes it from global
+// giving the same bits.  The 2D
+// candidate loop is branch-free FP32; a 3D window is tested by distance
+// first, and terms are formed for what that keeps.  A target that meets a
+// candidate needing the FP64 decision is deferred: its warp recomputes it from global
 // memory at the end (fixup_target).
 //
 // Pair test.  The reference keeps a pair when d2 != 0 && d2 <= rmax*rmax in
@@ -51,6 +52,8 @@
 // than 3 cells per axis, where the reference visits a cell more than once,
 // take the literal path (general_scan).
 #pragma once
+
+#include <type_traits>
 
 #include "force_common.cuh"
 
@@ -147,16 +150,15 @@ __global__ void __launch_bounds__(kThreads) k_force_general(const __grid_constan
 // windows overflow.  Few stencil cells keep variant 1 at 4 blocks per SM
 // (with 768 cells and 128 targets only 4 blocks of 4 warps fitted: 15%
 // slower on the batched worlds).
-// 3D: variant 0 (5 blocks of 128 targets at 96 registers) holds 71 staged
-// columns of 9 cells, so that the sparse tails of a blob world stage in one
-// or two rounds, and 2176 candidates for the dense cores (on the 4M-blob
-// world 1.41 ms per launch against 1.49 with 512 cells and 2048 candidates
-// and 1.45 with 384 and 2304; shapes whose shared memory leaves 4 blocks
-// per SM lose 5-10%); variant 1 is the smaller tile for sparse worlds.
+// 3D: variant 0 (4 blocks of 128 targets) holds 71 staged columns of 9 cells,
+// so that the sparse tails of a blob world stage in one or two rounds, and
+// 2176 candidates for the dense cores; variant 1 is the smaller tile for
+// sparse worlds.
 // Variant 2: 2D, 8 blocks of 128 targets with 256 cells and 1024 candidates,
 // for small worlds, which the 256-target tiles cut into too few blocks (the
-// 10k-particle world: 40 blocks of 256 on 152 SMs); 3D, 4 blocks of 128
-// targets with 2816 candidates, for dense worlds.
+// 10k-particle world: 40 blocks of 256 on 152 SMs); 3D, 5 blocks of 128
+// targets with 1728 candidates (4M blobs: force 1157 us against 1169 for
+// variant 0; 1M uniform with 50 neighbours: 359 against 323).
 template <int D, int V>
 struct TileCfg;
 template <>
@@ -173,16 +175,19 @@ struct TileCfg<2, 2> {
 };
 template <>
 struct TileCfg<3, 0> {
-    static constexpr int kTargets = 128, kMinBlocks = 5, kCap = 2176, kCells = 640;
+    static constexpr int kTargets = 128, kMinBlocks = 4, kCap = 2176, kCells = 640;
 };
 template <>
 struct TileCfg<3, 1> {
-    static constexpr int kTargets = 64, kMinBlocks = 10, kCap = 1024, kCells = 384;
+    static constexpr int kTargets = 64, kMinBlocks = 10, kCap = 832, kCells = 320;
 };
 template <>
 struct TileCfg<3, 2> {
-    static constexpr int kTargets = 128, kMinBlocks = 4, kCap = 2816, kCells = 640;
+    static constexpr int kTargets = 128, kMinBlocks = 5, kCap = 1728, kCells = 448;
 };
+
+// Words of 32 candidates a 3D target tests before it forms the kept terms.
+constexpr int kCullWords = 8;
 
 // Lives in dynamic shared memory (variant 0: about 28 KB in 2D, 42 KB in 3D).
 // Staged columns: the sorted union of the windows cx-1..cx+1 of the staged
@@ -191,13 +196,16 @@ struct TileCfg<3, 2> {
 template <int D, int V>
 struct TileSmem {
     static constexpr int kCols = TileCfg<D, V>::kCells / TileRows<D>::R;
-    float4 cand[TileCfg<D, V>::kCap];      // staged candidates, column-major by stencil cell
+    float4 cand[TileCfg<D, V>::kCap + (D == 3 ? 8 : 0)];  // staged candidates, column-major by stencil cell
     int coff[TileCfg<D, V>::kCells + 1];   // smem start of stencil cell e = column * R + row
     int cglob[TileCfg<D, V>::kCells];      // sorted-order start of stencil cell e
     int colv[kCols];                       // virtual column of staged column ci
     int colrow[kCols];                     // grid row of staged column ci: y, or y | z << 16
     int wsum[TileCfg<D, V>::kTargets / 32];
     int wcol[TileCfg<D, V>::kTargets / 32];
+    // 3D: the words of 32 candidates that keep some, thread t's k-th at
+    // [k * kTargets + t] (bits, staged index of bit 31)
+    uint2 kept[D == 3 ? (kCullWords + 1) * TileCfg<D, V>::kTargets : 1];
     float mat[kSmemMatrixMax * smem_matrix_stride<D>(kSmemMatrixMax)];
     uint8_t image[TileCfg<D, V>::kCells];  // image shifts of stencil cell e (kUp*, kDown*)
 };
@@ -451,34 +459,23 @@ __global__ void __launch_bounds__(TileCfg<D, V>::kTargets, TileCfg<D, V>::kMinBl
     const float* Mrow = M + (valid ? Layout<D>::type(me) : 0) * ms;
     Acc acc = {0.f, 0.f, 0.f, 0, 0ull, 0ull, 0ull};
     bool defer = false, direct = false;
-    // The target's window: staged columns k .. k+2; the target itself splits
+    // 2D.  The target's window: staged columns k .. k+2; the target itself splits
     // its run into [j0, self_j) and (self_j, j1).  Only a target in the last
-    // column, row or layer of a periodic box meets candidates flagged for a
+    // column or row of a periodic box meets candidates flagged for a
     // target shift.
-    auto evaluate = [&](int k, int ncell) {
+    auto evaluate2 = [&](int k, int ncell) {
         const int j0 = sm.coff[k * R], j1 = sm.coff[(k + 3) * R];
         const int own = (k + 1) * R + R / 2;
         const int self_j = sm.coff[own] + (s - sm.cglob[own]);
-        const bool shift = P.wrap && (cx == nx - 1 || cy == nx - 1 || (D == 3 && cz == nx - 1));
+        const bool shift = P.wrap && (cx == nx - 1 || cy == nx - 1);
         const int* co = sm.coff;
         const int* cg = sm.cglob;
-        // 2D: three runs, before the target's own cell, the own cell (the
-        // target itself neutralised in place), after it: every lane of a cell
-        // walks the same addresses, so the candidate loads are broadcasts
-        // (2.7% faster than splitting at the target).  3D: two runs split at
-        // the target (the three-run form measured 8% slower).  Same bits.
+        // Three runs, before the target's own cell, the own cell (the target
+        // itself neutralised in place), after it: every lane of a cell walks
+        // the same addresses, so the candidate loads are broadcasts (2.7%
+        // faster than splitting at the target).  Same bits.
         const int o0 = co[own], o1 = co[own + 1];
-        if (D == 3) {
-            if (shift) {
-                defer = cand_range<D, DBG, true>(A, P, sm.cand, co, cg, Mrow, ncell, j0, self_j, px, py, pz, acc);
-                defer |= cand_range<D, DBG, true>(A, P, sm.cand, co, cg, Mrow, ncell, self_j + 1, j1, px, py, pz,
-                                                  acc);
-            } else {
-                defer = cand_range<D, DBG, false>(A, P, sm.cand, co, cg, Mrow, ncell, j0, self_j, px, py, pz, acc);
-                defer |= cand_range<D, DBG, false>(A, P, sm.cand, co, cg, Mrow, ncell, self_j + 1, j1, px, py, pz,
-                                                   acc);
-            }
-        } else if (shift) {
+        if (shift) {
             defer = cand_range<D, DBG, true>(A, P, sm.cand, co, cg, Mrow, ncell, j0, o0, px, py, pz, acc);
             defer |= cand_range<D, DBG, true, true>(A, P, sm.cand, co, cg, Mrow, ncell, o0, o1, px, py, pz, acc,
                                                     self_j);
@@ -490,11 +487,91 @@ __global__ void __launch_bounds__(TileCfg<D, V>::kTargets, TileCfg<D, V>::kMinBl
             defer |= cand_range<D, DBG, false>(A, P, sm.cand, co, cg, Mrow, ncell, o1, j1, px, py, pz, acc);
         }
     };
+    // 3D, the whole warp together (a lane without `mine` takes no part):
+    // kCullWords words at a time, the distance test, then the kept
+    // candidates' terms.
+    auto evaluate3 = [&](bool mine, int k, int ncell) {
+        int j0 = 0, j1 = 0, self = -1;
+        if (mine) {
+            j0 = sm.coff[k * R];
+            j1 = sm.coff[(k + 3) * R];
+            const int own = (k + 1) * R + R / 2;
+            self = sm.coff[own] + (s - sm.cglob[own]);
+            if (DBG) acc.cand += j1 - j0 - 1;
+        }
+        const LoopK K(P);
+        const float neg_thr = -(float)P.rmax2 * (1.f + kCullRel);
+        float umin = INFINITY;
+        uint2* kept = sm.kept + tid;
+        auto walk = [&](auto shifted) {
+            constexpr bool kShifted = decltype(shifted)::value;
+            const float px1 = px - 1.f, py1 = py - 1.f, pz1 = pz - 1.f;
+            for (int j = j0; j < j1; j += 32 * kCullWords) {
+                const int nw = min(kCullWords, (j1 - j + 31) >> 5);
+                // The words that keep something, with the staged index of
+                // their bit 31, and how many candidates they keep.
+                uint2* put = kept;
+                int n = 0;
+                for (int i = 0; i < nw; ++i) {
+                    const int base = j + 32 * i;
+                    uint32_t m = cull_word<kShifted>(sm.cand + base, min(32, j1 - base), px, py, pz, neg_thr);
+                    if ((unsigned)(self - base) < 32u) m &= ~(0x80000000u >> (self - base));
+                    if (m) {
+                        *put = make_uint2(m, (uint32_t)base + 31);
+                        put += kT;
+                        n += __popc(m);
+                    }
+                }
+                uint2 next = kept[0];  // the word after the current one
+                const uint2* get = kept;
+                uint32_t m = 0, top = 0;
+                for (; n > 0; --n) {
+                    if (m == 0u) {
+                        m = next.x;
+                        top = next.y;
+                        get += kT;
+                        next = *get;
+                    }
+                    const int b = top_bit(m);
+                    m &= (1u << b) - 1u;
+                    const float4 q = sm.cand[top - b];
+                    int tb = __float_as_int(q.w);
+                    float pxe = px, pye = py, pze = pz;
+                    if (kShifted) {
+                        pxe = (tb & kShiftX) ? px1 : px;
+                        pye = (tb & kShiftY) ? py1 : py;
+                        pze = (tb & kShiftZ) ? pz1 : pz;
+                        tb &= 0xffff;
+                    }
+                    const Term<D> t = cand_term<D>(K, q.x, q.y, q.z, pxe, pye, pze, Mrow[tb], umin);
+                    add_term<D>(acc, t);
+                    if (DBG && (t.d2 <= K.lo) && t.d2 > 0.f)
+                        add_pair<D, true>(acc, make_float4(0.f, 0.f, 0.f, 0.f),
+                                          id_of<D>(A, staged_global(sm.coff, sm.cglob, ncell,
+                                                                    (int)(top - b))));
+                }
+            }
+        };
+        // Only a target in the last column, row or layer of a periodic box
+        // meets candidates flagged for a target shift.
+        if (__any_sync(kFull, mine && P.wrap && (cx == nx - 1 || cy == nx - 1 || cz == nx - 1)))
+            walk(std::true_type{});
+        else
+            walk(std::false_type{});
+        if (mine) defer = needs_fp64(K, umin);
+    };
+    auto evaluate = [&](bool mine, int k, int ncell) {
+        if constexpr (D == 3) {
+            evaluate3(mine, k, ncell);
+        } else {
+            if (mine) evaluate2(k, ncell);
+        }
+    };
     __syncthreads();
     const uint32_t* cs = A.cstart + P.cell_base;
     if (whole) {
         whole = stage_columns<D, V>(A, P, cs, sm, ncol);
-        if (whole && valid) evaluate(kwin, R * ncol);
+        if (whole) evaluate(valid, kwin, R * ncol);
     }
     if (!whole) {
         // Chunks of the block's window columns [a, hi), each serving the
@@ -513,7 +590,7 @@ __global__ void __launch_bounds__(TileCfg<D, V>::kTargets, TileCfg<D, V>::kMinBl
             const bool staged = stage_columns<D, V>(A, P, cs, sm, hi - a);
             const bool mine = valid && kwin >= a && kwin <= hi - 3;
             if (staged) {
-                if (mine) evaluate(kwin - a, R * (hi - a));
+                evaluate(mine, kwin - a, R * (hi - a));
                 a = hi - 2;
                 width = min(kCols, 2 * width);
             } else if (hi - a > 3) {
