@@ -17,6 +17,8 @@
 #include "plg_internal.cuh"
 #include "plgpu.h"
 
+#include <algorithm>
+
 namespace plg {
 
 namespace {
@@ -25,6 +27,11 @@ constexpr int kThreads = 256;
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 16;
 constexpr int kScanTile = kScanThreads * kScanItems;
+
+// k_sort_small: threads per block, slots a block is given (at most
+// kSmallBlocks blocks) and members its shared list holds.
+constexpr int kSmallThreads = 1024, kSmallShare = 512, kSmallBlocks = 128;
+constexpr uint32_t kSmallList = 4096;
 
 inline int blocks_for(int n, int threads) { return (n + threads - 1) / threads; }
 
@@ -431,6 +438,127 @@ __global__ void __launch_bounds__(kThreads) k_gather(int n, const uint32_t* __re
     if (cell_sorted) cell_sorted[st + r] = (int32_t)c;
 }
 
+// ---- the whole sort of a small world in one launch ----
+
+// k_scan, k_scatter and k_gather of a small world (sort_is_small) without
+// any exchange between blocks: every block counts all the cells from the
+// particles' cell indices in its own shared memory and scans them, then
+// sorts the cells whose first slot falls into its share of the slots.  A
+// small world's three launches are a chain of memory and launch latencies,
+// 3 to 4 us each however little they move; re-reading 4 bytes per particle
+// in every block costs less than handing results from block to block.
+template <int D>
+__global__ void __launch_bounds__(kSmallThreads) k_sort_small(int n, int ncells, const uint32_t* __restrict__ cell,
+                                                              uint32_t* __restrict__ counts,
+                                                              uint32_t* __restrict__ cstart, uint32_t* perm,
+                                                              uint32_t* __restrict__ slot_cell, StateBuf<D> a,
+                                                              StateBuf<D> b, int32_t* __restrict__ cell_sorted,
+                                                              uint32_t* zero_word) {
+    extern __shared__ uint32_t small_smem[];
+    uint32_t* const start = small_smem;              // first slot of each cell, ncells + 1
+    uint32_t* const next = start + ncells + 1;       // next free slot of each cell
+    uint32_t* const list = next + ncells;            // members of this block's slots
+    __shared__ uint32_t warp_sum[kSmallThreads / 32], own[2];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int all = blockIdx.x * kSmallThreads + tid, nall = gridDim.x * kSmallThreads;
+    pdl_release();
+    for (int c = tid; c < ncells; c += kSmallThreads) start[c] = 0u;
+    if (tid < 2) own[tid] = 0u;
+    __syncthreads();
+    pdl_wait();  // the force kernel's cells
+    if (zero_word && all == 0) *zero_word = 0u;  // the step's deferred-target count
+    for (int c = all; c < ncells; c += nall) counts[c] = 0u;  // for the next counting pass
+    // Four consecutive particles per thread: of one or two cells in a world
+    // that has been sorted before, so they count once or twice.
+    auto each4 = [&](auto f) {
+        for (int i = 4 * tid; i < n; i += 4 * kSmallThreads) {
+            uint4 q = make_uint4(0u, 0u, 0u, 0u);
+            const int m = min(4, n - i);
+            if (m == 4) {
+                q = *reinterpret_cast<const uint4*>(cell + i);
+            } else {
+                q.x = cell[i];
+                if (m > 1) q.y = cell[i + 1];
+                if (m > 2) q.z = cell[i + 2];
+            }
+            f(i, m, q);
+        }
+    };
+    each4([&](int, int m, uint4 q) {
+        uint32_t c = q.x, k = 1;
+        auto add = [&](uint32_t d) {
+            if (d == c) {
+                ++k;
+            } else {
+                atomicAdd(start + c, k);
+                c = d;
+                k = 1;
+            }
+        };
+        if (m > 1) add(q.y);
+        if (m > 2) add(q.z);
+        if (m > 3) add(q.w);
+        atomicAdd(start + c, k);
+    });
+    __syncthreads();
+    // Exclusive scan of the counts in place, an odd number of cells per
+    // thread (no bank conflicts); the cell holding a boundary of this block's
+    // share of the slots tells where its own slots begin and end.
+    const int per = ((ncells + kSmallThreads - 1) / kSmallThreads) | 1;
+    const int c0 = min(tid * per, ncells), c1 = min(c0 + per, ncells);
+    uint32_t sum = 0;
+    for (int c = c0; c < c1; ++c) sum += start[c];
+    const uint32_t inc = warp_inclusive(sum);
+    if (lane == 31) warp_sum[warp] = inc;
+    __syncthreads();
+    if (warp == 0) {
+        const uint32_t s = warp_sum[lane];
+        warp_sum[lane] = warp_inclusive(s) - s;
+    }
+    __syncthreads();
+    const uint32_t lo = (uint32_t)((int64_t)n * blockIdx.x / gridDim.x);
+    const uint32_t hi = (uint32_t)((int64_t)n * (blockIdx.x + 1) / gridDim.x);
+    uint32_t run = warp_sum[warp] + inc - sum;
+    for (int c = c0; c < c1; ++c) {
+        const uint32_t end = run + start[c];
+        start[c] = run;
+        next[c] = run;
+        if (run < lo && lo <= end) own[0] = end;
+        if (run < hi && hi <= end) own[1] = end;
+        run = end;
+    }
+    if (tid == 0) start[ncells] = (uint32_t)n;
+    __syncthreads();
+    const uint32_t own0 = own[0], own1 = own[1];
+    // The members of the block's cells, in any order within a cell; where
+    // they exceed the shared list, in the block's slots of perm.
+    uint32_t* const mem = own1 - own0 <= kSmallList ? list - own0 : perm;
+    each4([&](int i, int m, uint4 q) {
+        auto take = [&](int k, uint32_t c) {
+            if (k < m && start[c] >= lo && start[c] < hi) mem[atomicAdd(next + c, 1u)] = (uint32_t)(i + k);
+        };
+        take(0, q.x);
+        take(1, q.y);
+        take(2, q.z);
+        take(3, q.w);
+    });
+    __syncthreads();
+    // Stable order within the cell: the members of a smaller index go first.
+    for (uint32_t s = own0 + tid; s < own1; s += kSmallThreads) {
+        const uint32_t i = mem[s], c = cell[i];
+        const float4 p = a.pt[i];
+        const typename Layout<D>::Vel v = a.vel[i];
+        const uint32_t st = start[c], en = start[c + 1];
+        uint32_t r = 0;
+        for (uint32_t t = st; t < en; ++t) r += mem[t] < i ? 1u : 0u;
+        slot_cell[s] = c;
+        b.pt[st + r] = p;
+        b.vel[st + r] = v;
+        if (cell_sorted) cell_sorted[st + r] = (int32_t)c;
+    }
+    for (int c = all; c <= ncells; c += nall) cstart[c] = start[c];
+}
+
 }  // namespace
 
 inline bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
@@ -502,6 +630,38 @@ void launch_scatter(cudaStream_t st, int n, const uint32_t* cell, uint32_t* coun
     launch_after(k_scatter, dim3(blocks_for(n, kThreads * kScatterPer)), dim3(kThreads), 0, st, n, cell, counts,
                  cstart, perm, slot_cell, zero_state, nzero);
 }
+
+bool sort_is_small(int n, int ncells) { return n > 0 && n <= kSmallParticles && ncells <= kSmallCells; }
+
+namespace {
+size_t small_sort_smem(int ncells) { return sizeof(uint32_t) * (2 * (size_t)ncells + 1 + kSmallList); }
+}  // namespace
+
+template <int D>
+void launch_sort_small(cudaStream_t st, int n, int ncells, const uint32_t* cell, uint32_t* counts, uint32_t* cstart,
+                       uint32_t* perm, uint32_t* slot_cell, StateBuf<D> a, StateBuf<D> b, int32_t* cell_sorted,
+                       uint32_t* zero_word, bool after) {
+    const dim3 grid(std::min(kSmallBlocks, blocks_for(n, kSmallShare))), block(kSmallThreads);
+    const size_t smem = small_sort_smem(ncells);
+    if (after)
+        launch_after(k_sort_small<D>, grid, block, smem, st, n, ncells, cell, counts, cstart, perm, slot_cell, a, b,
+                     cell_sorted, zero_word);
+    else
+        k_sort_small<D><<<grid, block, smem, st>>>(n, ncells, cell, counts, cstart, perm, slot_cell, a, b, cell_sorted,
+                                                   zero_word);
+}
+
+cudaError_t sort_kernels_init() {
+    const int bytes = (int)small_sort_smem(kSmallCells);
+    const cudaError_t e = cudaFuncSetAttribute(k_sort_small<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(k_sort_small<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
+
+template void launch_sort_small<2>(cudaStream_t, int, int, const uint32_t*, uint32_t*, uint32_t*, uint32_t*, uint32_t*,
+                                   StateBuf<2>, StateBuf<2>, int32_t*, uint32_t*, bool);
+template void launch_sort_small<3>(cudaStream_t, int, int, const uint32_t*, uint32_t*, uint32_t*, uint32_t*, uint32_t*,
+                                   StateBuf<3>, StateBuf<3>, int32_t*, uint32_t*, bool);
 
 template <int D>
 void launch_gather(cudaStream_t st, int n, const uint32_t* perm, const uint32_t* slot_cell, const uint32_t* cstart,

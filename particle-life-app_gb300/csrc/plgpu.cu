@@ -324,18 +324,25 @@ void enqueue_body(plg_ctx* c, const DebugOut* dbg, int32_t* cell_sorted, const H
     // scatter sets it back after each scan; with no particles there is no
     // scatter, and a memset does it.
     const int nstate = c->nparts + 1;
+    uint32_t* const zero_word = c->general ? nullptr : c->defer;
+    const bool small = sort_is_small(n, c->ncells);
     k0(PLG_K_SCAN);
-    launch_scan(st, c->counts, c->ncells, c->cstart, c->scan_state, c->status_d, c->general ? nullptr : c->defer,
-                !c->profiling);
+    if (small)  // the whole sort (profiled as the scan)
+        launch_sort_small<D>(st, n, c->ncells, c->cell, c->counts, c->cstart, c->perm, c->slot_cell, buf_a<D>(c),
+                             buf_b<D>(c), cell_sorted, zero_word, !c->profiling);
+    else
+        launch_scan(st, c->counts, c->ncells, c->cstart, c->scan_state, c->status_d, zero_word, !c->profiling);
     k1(PLG_K_SCAN);
     k0(PLG_K_SCATTER);
-    if (n > 0)
-        launch_scatter(st, n, c->cell, c->counts, c->cstart, c->perm, c->slot_cell, c->scan_state, nstate);
-    else
-        cudaMemsetAsync(c->scan_state, 0, sizeof(unsigned long long) * (size_t)nstate, st);
+    if (!small) {
+        if (n > 0)
+            launch_scatter(st, n, c->cell, c->counts, c->cstart, c->perm, c->slot_cell, c->scan_state, nstate);
+        else
+            cudaMemsetAsync(c->scan_state, 0, sizeof(unsigned long long) * (size_t)nstate, st);
+    }
     k1(PLG_K_SCATTER);
     k0(PLG_K_GATHER);
-    launch_gather<D>(st, n, c->perm, c->slot_cell, c->cstart, buf_a<D>(c), buf_b<D>(c), cell_sorted);
+    if (!small) launch_gather<D>(st, n, c->perm, c->slot_cell, c->cstart, buf_a<D>(c), buf_b<D>(c), cell_sorted);
     k1(PLG_K_GATHER);
     k0(PLG_K_FORCE);
     launch_force<D>(st, c->fp, c->general, buf_b<D>(c), c->cstart, c->slot_cell, buf_a<D>(c), c->cell, c->counts,
@@ -554,7 +561,7 @@ int plg_create(int dim, int64_t capacity, plg_ctx** out) {
     const size_t cap = (size_t)capacity;
     e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) rc = PLG_E_CUDA;
-    if (!rc && force_kernels_init() != cudaSuccess) rc = PLG_E_CUDA;
+    if (!rc && (force_kernels_init() != cudaSuccess || sort_kernels_init() != cudaSuccess)) rc = PLG_E_CUDA;
     dmalloc((void**)&c->apt, sizeof(float4) * cap);
     dmalloc((void**)&c->bpt, sizeof(float4) * cap);
     dmalloc(&c->avel, vel_sz * cap);
