@@ -7,6 +7,7 @@
 #pragma once
 
 #include <climits>
+#include <type_traits>
 
 #include "plg_internal.cuh"
 
@@ -528,31 +529,38 @@ __device__ __forceinline__ int staged_global(const int* coff, const int* cglob, 
     return cglob[lo] + (j - coff[lo]);
 }
 
-// Staged candidates [ja, jb) of the target (a part of its neighbourhood
-// without the target itself), from a column-major staging (cand, with cell
-// offsets coff and global starts cglob of ncell cells).  Branch-free FP32:
-// every lane evaluates the Accelerator for every candidate, and a pair
-// beyond rmax adds an exact zero (eval_candidate).  A candidate that needs
-// the FP64 decision (the |u| test of LoopK: the decision band around rmax,
-// coincident particles) makes the function return true: the caller then
-// defers the target to the FP64 fixup, which discards this partial sum.
+// 2D: the staged candidates [j0, j1) of a target, itself at self_j among the
+// members [o0, o1) of its own cell, from a column-major staging (cand, with
+// cell offsets coff and global starts cglob of ncell cells).  Branch-free
+// FP32: every lane evaluates the Accelerator for every candidate, and a pair
+// beyond rmax adds an exact zero (cand_term).  The target's own copy is moved
+// 8 units away (an exact zero term, far from both zeros of u), which sums to
+// the same bits as leaving it out.  A candidate that needs the FP64 decision
+// (the |u| test of LoopK: the decision band around rmax, coincident
+// particles) makes the function return true: the caller then defers the
+// target to the FP64 fixup, which discards this partial sum.
 // SHIFT: some candidates carry target-shift flags.
-// SELF: the range holds the target itself at self_j; its copy is moved 8
-// units away (an exact zero term, far from both zeros of u), which sums to
-// the same bits as leaving it out, without a branch.
-template <int D, bool DBG, bool SHIFT, bool SELF = false>
-__device__ __forceinline__ bool cand_range(const ForceArgs<D>& A, const ForceParams& P, const float4* cand,
-                                           const int* coff, const int* cglob, const float* __restrict__ Mrow,
-                                           int ncell, int ja, int jb, float px, float py, float pz, Acc& acc,
-                                           int self_j = -1) {
+//
+// Four candidates per iteration: their terms are independent chains
+// (shared-memory load, rsqrt, force law) that overlap in one warp; they are
+// added in candidate order, so the sum has the same bits as one candidate at
+// a time.  Only the iterations over the own cell look for the target; they
+// take the odd candidates before and after it with them, so that a window
+// has one remainder instead of one before, in and after the cell.  Every
+// lane of a cell walks the same addresses: the loads are broadcasts.
+template <int D, bool DBG, bool SHIFT>
+__device__ __forceinline__ bool cand_window(const ForceArgs<D>& A, const ForceParams& P, const float4* cand,
+                                            const int* coff, const int* cglob, const float* __restrict__ Mrow,
+                                            int ncell, int j0, int o0, int o1, int j1, int self_j, float px, float py,
+                                            float pz, Acc& acc) {
     const float px1 = px - 1.f, py1 = py - 1.f, pz1 = pz - 1.f;
     float umin = INFINITY;
     const LoopK K(P);
     // The term of candidate j, with the staged shifts applied.
-    auto term = [&](int j) {
+    auto term = [&](auto self, int j) {
         float4 q = cand[j];
-        if (SELF && j == self_j) q.x += 8.f;
-        int tb = __float_as_int(D == 3 ? q.w : q.z);
+        if (decltype(self)::value && j == self_j) q.x += 8.f;
+        int tb = Layout<D>::type(q);
         float pxe = px, pye = py, pze = pz;
         if (SHIFT) {
             pxe = (tb & kShiftX) ? px1 : px;
@@ -563,32 +571,31 @@ __device__ __forceinline__ bool cand_range(const ForceArgs<D>& A, const ForcePar
         return cand_term<D>(K, q.x, q.y, q.z, pxe, pye, pze, Mrow[tb], umin);
     };
     auto count = [&](int j, float d2) {
-        if (DBG && !(SELF && j == self_j)) {
+        if (DBG && j != self_j) {
             acc.cand++;
             if ((d2 <= K.lo) & (d2 > 0.f))
                 add_pair<D, true>(acc, make_float4(0.f, 0.f, 0.f, 0.f),
                                   id_of<D>(A, staged_global(coff, cglob, ncell, j)));
         }
     };
-    // Two candidates per iteration: their terms are independent chains
-    // (shared-memory load, rsqrt, force law) that overlap in one warp; they
-    // are added in candidate order, so the sum has the same bits as one
-    // candidate at a time.
-    constexpr int U = 2;
-    int j = ja;
-    for (; j + U <= jb; j += U) {
+    constexpr int U = 4;
+    auto four = [&](auto self, int j) {
         Term<D> t[U];
 #pragma unroll
-        for (int k = 0; k < U; ++k) t[k] = term(j + k);
+        for (int k = 0; k < U; ++k) t[k] = term(self, j + k);
 #pragma unroll
         for (int k = 0; k < U; ++k) add_term<D>(acc, t[k]);
 #pragma unroll
         for (int k = 0; k < U; ++k) count(j + k, t[k].d2);
-    }
-    for (; j < jb; ++j) {
-        const Term<D> t0 = term(j);
-        add_term<D>(acc, t0);
-        count(j, t0.d2);
+    };
+    int j = j0;
+    for (; j + U <= o0; j += U) four(std::false_type{}, j);
+    for (; j < o1 && j + U <= j1; j += U) four(std::true_type{}, j);
+    for (; j + U <= j1; j += U) four(std::false_type{}, j);
+    for (; j < j1; ++j) {
+        const Term<D> t = term(std::true_type{}, j);
+        add_term<D>(acc, t);
+        count(j, t.d2);
     }
     return needs_fp64(K, umin);
 }

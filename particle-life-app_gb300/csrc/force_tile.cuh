@@ -53,8 +53,6 @@
 // take the literal path (general_scan).
 #pragma once
 
-#include <type_traits>
-
 #include "force_common.cuh"
 
 namespace plg {
@@ -449,43 +447,25 @@ __global__ void __launch_bounds__(TileCfg<D, V>::kTargets, TileCfg<D, V>::kMinBl
             }
         }
     };
-    constexpr int kCols = TileSmem<D, V>::kCols;
-    // One staging for the whole block when every window fits; otherwise in
-    // chunks of columns (below).
-    bool whole = ncol <= kCols;  // block-uniform
-    if (whole) fill_columns(0, ncol);
     const int nx = P.g.nx;
     const float px = me.x, py = me.y, pz = D == 3 ? me.z : 0.f;
     const float* Mrow = M + (valid ? Layout<D>::type(me) : 0) * ms;
     Acc acc = {0.f, 0.f, 0.f, 0, 0ull, 0ull, 0ull};
     bool defer = false, direct = false;
-    // 2D.  The target's window: staged columns k .. k+2; the target itself splits
-    // its run into [j0, self_j) and (self_j, j1).  Only a target in the last
-    // column or row of a periodic box meets candidates flagged for a
-    // target shift.
-    auto evaluate2 = [&](int k, int ncell) {
+    // 2D, the whole warp together (a lane without `mine` takes no part).  The
+    // target's window: staged columns k .. k+2.  Only a target in the last
+    // column or row of a periodic box meets candidates flagged for a target
+    // shift; its whole warp then heeds the flags.
+    auto evaluate2 = [&](bool mine, int k, int ncell) {
+        const bool any_shift = __any_sync(kFull, mine && P.wrap && (cx == nx - 1 || cy == nx - 1));
+        if (!mine) return;
         const int j0 = sm.coff[k * R], j1 = sm.coff[(k + 3) * R];
-        const int own = (k + 1) * R + R / 2;
-        const int self_j = sm.coff[own] + (s - sm.cglob[own]);
-        const bool shift = P.wrap && (cx == nx - 1 || cy == nx - 1);
-        const int* co = sm.coff;
-        const int* cg = sm.cglob;
-        // Three runs, before the target's own cell, the own cell (the target
-        // itself neutralised in place), after it: every lane of a cell walks
-        // the same addresses, so the candidate loads are broadcasts (2.7%
-        // faster than splitting at the target).  Same bits.
-        const int o0 = co[own], o1 = co[own + 1];
-        if (shift) {
-            defer = cand_range<D, DBG, true>(A, P, sm.cand, co, cg, Mrow, ncell, j0, o0, px, py, pz, acc);
-            defer |= cand_range<D, DBG, true, true>(A, P, sm.cand, co, cg, Mrow, ncell, o0, o1, px, py, pz, acc,
-                                                    self_j);
-            defer |= cand_range<D, DBG, true>(A, P, sm.cand, co, cg, Mrow, ncell, o1, j1, px, py, pz, acc);
-        } else {
-            defer = cand_range<D, DBG, false>(A, P, sm.cand, co, cg, Mrow, ncell, j0, o0, px, py, pz, acc);
-            defer |= cand_range<D, DBG, false, true>(A, P, sm.cand, co, cg, Mrow, ncell, o0, o1, px, py, pz, acc,
-                                                     self_j);
-            defer |= cand_range<D, DBG, false>(A, P, sm.cand, co, cg, Mrow, ncell, o1, j1, px, py, pz, acc);
-        }
+        const int own = (k + 1) * R + R / 2, o0 = sm.coff[own], o1 = sm.coff[own + 1];
+        const int self_j = o0 + (s - sm.cglob[own]);
+        defer = any_shift ? cand_window<D, DBG, true>(A, P, sm.cand, sm.coff, sm.cglob, Mrow, ncell, j0, o0, o1, j1,
+                                                      self_j, px, py, pz, acc)
+                          : cand_window<D, DBG, false>(A, P, sm.cand, sm.coff, sm.cglob, Mrow, ncell, j0, o0, o1, j1,
+                                                       self_j, px, py, pz, acc);
     };
     // 3D, the whole warp together (a lane without `mine` takes no part):
     // kCullWords words at a time, the distance test, then the kept
@@ -561,44 +541,37 @@ __global__ void __launch_bounds__(TileCfg<D, V>::kTargets, TileCfg<D, V>::kMinBl
         if (mine) defer = needs_fp64(K, umin);
     };
     auto evaluate = [&](bool mine, int k, int ncell) {
-        if constexpr (D == 3) {
+        if constexpr (D == 3)
             evaluate3(mine, k, ncell);
-        } else {
-            if (mine) evaluate2(k, ncell);
-        }
+        else
+            evaluate2(mine, k, ncell);
     };
-    __syncthreads();
     const uint32_t* cs = A.cstart + P.cell_base;
-    if (whole) {
-        whole = stage_columns<D, V>(A, P, cs, sm, ncol);
-        if (whole) evaluate(valid, kwin, R * ncol);
-    }
-    if (!whole) {
-        // Chunks of the block's window columns [a, hi), each serving the
-        // targets whose window starts in [a, hi - 3].  A chunk may span
-        // segments: its columns are staged one by one with their own rows,
-        // and a window never leaves its segment.  A chunk whose candidates do
-        // not fit is retried with half as many columns (the width grows back
-        // after a success), and a single window that does not fit is read
-        // from global memory.  (Per-segment chunks served one segment per
-        // staging round: sparse 3D blocks spread over many grid rows.)
-        int a = 0, width = kCols;
-        while (a <= ncol - 3) {
-            const int hi = min(a + width, ncol);
-            fill_columns(a, hi);  // the previous staging no longer reads the columns
-            __syncthreads();
-            const bool staged = stage_columns<D, V>(A, P, cs, sm, hi - a);
-            const bool mine = valid && kwin >= a && kwin <= hi - 3;
-            if (staged) {
-                evaluate(mine, kwin - a, R * (hi - a));
-                a = hi - 2;
-                width = min(kCols, 2 * width);
-            } else if (hi - a > 3) {
-                width = max(3, (hi - a) / 2);
-            } else {
-                if (mine) direct = true;  // computed after the loop, off the hot path
-                a += 1;
-            }
+    // Stagings of the block's window columns [a, hi), each serving the
+    // targets whose window starts in [a, hi - 3]; one staging serves them all
+    // when every window fits.  A staging may span segments: its columns are
+    // staged one by one with their own rows, and a window never leaves its
+    // segment.  A staging whose candidates do not fit is retried with half as
+    // many columns (the width grows back after a success), and a single
+    // window that does not fit is read from global memory.  (Per-segment
+    // stagings served one segment per round: sparse 3D blocks spread over
+    // many grid rows.)
+    constexpr int kCols = TileSmem<D, V>::kCols;
+    for (int a = 0, width = kCols; a <= ncol - 3;) {
+        const int hi = min(a + width, ncol);
+        fill_columns(a, hi);  // the previous staging no longer reads the columns
+        __syncthreads();
+        const bool staged = stage_columns<D, V>(A, P, cs, sm, hi - a);
+        const bool mine = valid && kwin >= a && kwin <= hi - 3;
+        if (staged) {
+            evaluate(mine, kwin - a, R * (hi - a));
+            a = hi - 2;
+            width = min(kCols, 2 * width);
+        } else if (hi - a > 3) {
+            width = max(3, (hi - a) / 2);
+        } else {
+            if (mine) direct = true;  // computed after the loop, off the hot path
+            a += 1;
         }
     }
     if (direct) {
