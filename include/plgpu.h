@@ -301,7 +301,8 @@ int plg_set_use_graph(plg_ctx* ctx, int32_t on);
 
 /* Force kernel tile variant of this world (see PLG_TILE_VARIANTS below).
  * Until plg_set_tile or plg_autotune chooses one, 2D worlds under 300,000
- * particles use variant 2 and all others variant 0.  Every variant gives
+ * particles use variant 2 and all others variant 0, except crowded 2D worlds
+ * (48 particles per cell or more on average): variant 1.  Every variant gives
  * the same bits. */
 int plg_set_tile(plg_ctx* ctx, int32_t variant);
 int plg_get_tile(plg_ctx* ctx, int32_t* variant);
@@ -424,9 +425,11 @@ int plg_batch_get_stream(plg_batch* batch, void** stream);
 const char* plg_batch_last_error(plg_batch* batch);
 int plg_batch_step_stats(plg_batch* batch, int64_t* deferred);
 /* Force kernel tile variants (threads = targets per block, staging size):
- * 2D: 0 = 256 targets / 1536 staged candidates, 1 = 256 / 3072 (dense
- * worlds), 2 = 128 / 1024 (small worlds); 3D: 0 = 128 / 2176, 1 = 64 / 832
- * (sparse worlds), 2 = 128 / 1728 (more blocks per SM).  All give the same bits.  Each world
+ * 2D: 0 = 128 targets / 1152 staged candidates, 1 = 128 / 2048 (crowded
+ * worlds), 2 = 128 / 1280 with more registers (small worlds); 3D: 0 = 128 /
+ * 2176, 1 = 64 / 832 (sparse worlds), 2 = 128 / 1728 (more blocks per SM).
+ * All give the same bits.  Until a variant is set or tuned, a world joins
+ * with variant 0, or 1 when it is a crowded 2D world (plg_set_tile).  Each world
  * of a batch has its own variant; a step launches the force kernel once per
  * variant in use.  The cell size is not a tuning choice: it is rmax (the
  * sorted order the reference exposes depends on it).  A single world has

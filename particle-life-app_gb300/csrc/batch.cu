@@ -111,6 +111,7 @@ struct plg_batch {
     int64_t side_stage_cap = 0;
     int32_t next_id = 1;
     int variant = 0;  // tile variant given to new worlds (plg_batch_set_tile sets every world's)
+    bool variant_auto = true;  // neither set nor tuned: crowded worlds get the dense tile
     unsigned long long* wcycles_d = nullptr;  // wcap: per-world block cycles (per-world autotuner)
     void* tune_save[5] = {};                  // the tuners' copy of the state (kept, grown on demand)
     size_t tune_cap[5] = {};
@@ -278,6 +279,11 @@ int check_desc(plg_batch* b, const plg_world_desc& d) {
     return rc ? berr(b, rc, msg) : PLG_OK;
 }
 
+// The tile variant of a world that joins.
+int new_world_variant(const plg_batch* b, const WorldRec& w) {
+    return b->variant_auto && crowded_world(b->dim, w.n, w.ncells) ? 1 : b->variant;
+}
+
 // The force kernel's tile tables: for each variant v, the first tile of
 // every world in the launch of v's worlds (a world of another variant has
 // no tiles there).  A block never spans two worlds, and every world is cut
@@ -392,12 +398,12 @@ int relayout(plg_batch* b, const std::vector<int>& survivors, const plg_world_de
         const plg_world_desc& d = add[a];
         WorldRec w;
         w.id = b->next_id++;
-        w.variant = b->variant;
         w.n = d.n;
         w.ntypes = d.ntypes;
         w.s = d.settings;
         w.nx = grid_n(d.settings.rmax);
         w.ncells = (int64_t)w.nx * w.nx * (D == 3 ? w.nx : 1);
+        w.variant = new_world_variant(b, w);
         w.bounds.resize((size_t)w.nx + 1);
         build_bounds(d.settings.rmax, w.nx, w.bounds.data());
         w.matrix.resize((size_t)d.ntypes * d.ntypes);
@@ -614,12 +620,12 @@ template <int D>
 int append_world(plg_batch* b, const plg_world_desc& d, const WorldGen* gen, int32_t steps, cudaStream_t side,
                  int32_t* id_out) {
     WorldRec w;
-    w.variant = b->variant;
     w.n = d.n;
     w.ntypes = d.ntypes;
     w.s = d.settings;
     w.nx = grid_n(d.settings.rmax);
     w.ncells = (int64_t)w.nx * w.nx * (D == 3 ? w.nx : 1);
+    w.variant = new_world_variant(b, w);
     const int64_t nbounds = w.nx + 1, nmat = (int64_t)d.ntypes * d.ntypes;
     if (b->n_total + b->pend_n + w.n > b->pcap) return berr(b, PLG_E_CAPACITY, "batch particle capacity exceeded");
     if (b->c_total + b->pend_c + w.ncells > b->ccap) return berr(b, PLG_E_CAPACITY, "batch cell capacity exceeded");
@@ -1061,6 +1067,7 @@ int plg_batch_set_tile(plg_batch* b, int32_t variant) {
     if (variant < 0 || variant >= PLG_TILE_VARIANTS) return berr(b, PLG_E_INVALID_ARG, "unknown tile variant");
     BatchDeviceGuard g(b->device);
     b->variant = variant;
+    b->variant_auto = false;
     for (WorldRec& w : b->worlds) w.variant = variant;
     for (WorldRec& w : b->pending) w.variant = variant;
     return write_tiles(b);
@@ -1226,6 +1233,7 @@ int plg_batch_autotune(plg_batch* b, int32_t steps, int32_t* chosen, double* ms_
     }
     best_v = switch_if_faster(old, best_v, times);
     b->variant = best_v;
+    b->variant_auto = false;
     set_all_variants(b, best_v);
     if (chosen) *chosen = best_v;
     return write_tiles(b);

@@ -139,37 +139,32 @@ __global__ void __launch_bounds__(kThreads) k_force_general(const __grid_constan
 //               blocks with spilled registers measured slower)
 //   kCap        staged candidates per staging
 //   kCells      stencil cells per staging (R x columns)
-// 2D: both variants are 4 blocks of 256 targets per SM at 64 registers
-// (32 warps) with 192 stencil cells (64 columns) per staging.  Variant 0
-// stages 1536 candidates (28 KB of shared memory) and suits sparse worlds
-// such as the 1M-particle one (95 us per launch against 97 for 8 blocks of
-// 128 targets with 256 cells); variant 1 stages 3072 (53 KB) for dense
-// worlds (tens to hundreds of particles per cell), where variant 0's
-// windows overflow.  Few stencil cells keep variant 1 at 4 blocks per SM
-// (with 768 cells and 128 targets only 4 blocks of 4 warps fitted: 15%
-// slower on the batched worlds).
+// 2D: tiles of 128 targets throughout (256 at 4 blocks per SM lose 2% at 6
+// particles per cell and 30% at 3 and below, where their windows need more
+// than the 256 stencil cells).  Variant 0: 8 blocks at 64 registers.  Variant
+// 1: 2048 candidates at 6 blocks for crowded cells (400k particles, 119 per
+// cell: 330 us against 498, 60 per cell: 169 against 172).  Variant 2: 7
+// blocks with more registers and candidates, for worlds of about one wave.
 // 3D: variant 0 (4 blocks of 128 targets) holds 71 staged columns of 9 cells,
 // so that the sparse tails of a blob world stage in one or two rounds, and
 // 2176 candidates for the dense cores; variant 1 is the smaller tile for
 // sparse worlds.
-// Variant 2: 2D, 8 blocks of 128 targets with 256 cells and 1024 candidates,
-// for small worlds, which the 256-target tiles cut into too few blocks (the
-// 10k-particle world: 40 blocks of 256 on 152 SMs); 3D, 5 blocks of 128
+// 3D variant 2: 5 blocks of 128
 // targets with 1728 candidates (4M blobs: force 1157 us against 1169 for
 // variant 0; 1M uniform with 50 neighbours: 359 against 323).
 template <int D, int V>
 struct TileCfg;
 template <>
 struct TileCfg<2, 0> {
-    static constexpr int kTargets = 256, kMinBlocks = 4, kCap = 1536, kCells = 192;
+    static constexpr int kTargets = 128, kMinBlocks = 8, kCap = 1152, kCells = 256;
 };
 template <>
 struct TileCfg<2, 1> {
-    static constexpr int kTargets = 256, kMinBlocks = 4, kCap = 3072, kCells = 192;
+    static constexpr int kTargets = 128, kMinBlocks = 6, kCap = 2048, kCells = 128;
 };
 template <>
 struct TileCfg<2, 2> {
-    static constexpr int kTargets = 128, kMinBlocks = 8, kCap = 1024, kCells = 256;
+    static constexpr int kTargets = 128, kMinBlocks = 7, kCap = 1280, kCells = 256;
 };
 template <>
 struct TileCfg<3, 0> {

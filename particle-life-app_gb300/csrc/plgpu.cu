@@ -297,14 +297,15 @@ void compute_force_params(plg_ctx* c) {
 
 Grid grid_of(plg_ctx* c) { return c->fp.g; }
 
-// 2D worlds below this many particles default to tile variant 2 (128
-// targets per block): with the 256-target variant 0 they fill fewer than
-// two waves of blocks (10k particles: 20.7 against 25.0 us per step).
+// 2D worlds below this many particles default to tile variant 2: they fill
+// at most two waves of blocks, and its extra registers count for more than
+// variant 0's eighth block.
 constexpr int64_t kSmallWorld2D = 300000;
 
 // The tile variant a step uses: the one set or tuned, else by size.
 int tile_variant(const plg_ctx* c) {
     if (!c->variant_auto) return c->variant;
+    if (crowded_world(c->dim, c->n, c->ncells)) return 1;
     return c->dim == 2 && c->n < kSmallWorld2D ? 2 : 0;
 }
 
