@@ -276,8 +276,8 @@ struct SplatParams {
     float size;
     int wrap;
 };
-int splat_samples_per_pixel();
-// winner: width * height * splat_samples_per_pixel() words of scratch;
+int splat_words_per_pixel();
+// winner: width * height * splat_words_per_pixel() words of scratch;
 // palette: ncolors RGBA floats (device); out: width * height RGBA8 (device).
 template <int D>
 void launch_splat(cudaStream_t st, int n, const float4* pt, const SplatParams& S, uint32_t* winner,
