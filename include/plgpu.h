@@ -121,7 +121,8 @@ int plg_upload(plg_ctx* ctx, int64_t n, const double* pos, const double* vel,
                const int32_t* type);
 
 /* nsteps x Physics.update() (Physics.java:112-134).  Blocks until done.
- * Checks the stop flag between steps: a set flag ends the call early with
+ * Checks the stop flag between steps (every fourth step in long calls on
+ * worlds of up to 524,288 particles): a set flag ends the call early with
  * PLG_E_STOPPED and is cleared (Physics.forceUpdateStop, Physics.java:149). */
 int plg_step(plg_ctx* ctx, int32_t nsteps);
 
