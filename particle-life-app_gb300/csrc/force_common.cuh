@@ -618,6 +618,8 @@ __device__ __forceinline__ bool cand_window(const ForceArgs<D>& A, const ForcePa
 // in blobs 1187 -> 1169 us, of 1M with 50 neighbours 416 -> 323 us.)
 constexpr float kCullRel = 1.6e-5f;
 
+constexpr int kCullGroup = 16;  // candidates per trip of the test (8: 2% slower, 32: the same)
+
 // Position of the highest set bit (m != 0).
 __device__ __forceinline__ int top_bit(uint32_t m) {
     int b;
@@ -627,16 +629,16 @@ __device__ __forceinline__ int top_bit(uint32_t m) {
 
 // Bit 31 - c: candidate c of the n <= 32 from `cand` on is kept for the
 // target at (px, py, pz).  SHIFT: some of them carry target-shift flags.
-// Reads whole groups of 8 (the staging is padded by that much).
+// Reads whole groups of kCullGroup (the staging is padded by that much).
 template <bool SHIFT>
 __device__ __forceinline__ uint32_t cull_word(const float4* __restrict__ cand, int n, float px, float py, float pz,
                                               float neg_thr) {
     const float px1 = px - 1.f, py1 = py - 1.f, pz1 = pz - 1.f;
     uint32_t m = 0;
     int c = 0;
-    for (; c < n; c += 8) {
+    for (; c < n; c += kCullGroup) {
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
+        for (int u = 0; u < kCullGroup; ++u) {
             const float4 q = cand[c + u];
             float pxe = px, pye = py, pze = pz;
             if (SHIFT) {

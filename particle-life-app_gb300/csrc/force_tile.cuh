@@ -189,7 +189,8 @@ constexpr int kCullWords = 8;
 template <int D, int V>
 struct TileSmem {
     static constexpr int kCols = TileCfg<D, V>::kCells / TileRows<D>::R;
-    float4 cand[TileCfg<D, V>::kCap + (D == 3 ? 8 : 0)];  // staged candidates, column-major by stencil cell
+    float4 before[D == 3 ? 8 : 1];         // read by the 3D distance test, never kept
+    float4 cand[TileCfg<D, V>::kCap + (D == 3 ? kCullGroup : 0)];  // staged candidates, column-major by stencil cell
     int coff[TileCfg<D, V>::kCells + 1];   // smem start of stencil cell e = column * R + row
     int cglob[TileCfg<D, V>::kCells];      // sorted-order start of stencil cell e
     int colv[kCols];                       // virtual column of staged column ci
@@ -414,6 +415,7 @@ __global__ void __launch_bounds__(TileCfg<D, V>::kTargets, TileCfg<D, V>::kMinBl
     const int pcol = tid > 0 ? pcx : 0;
     const bool start = valid && (tid == 0 || prow != row);
     const bool lead = valid && (start || pcol != cx);
+    const unsigned leads = __ballot_sync(kFull, lead);
     const int newc = !lead ? 0 : (start ? 3 : min(3, cx - pcol));
     int incl = newc;
 #pragma unroll
@@ -474,6 +476,11 @@ __global__ void __launch_bounds__(TileCfg<D, V>::kTargets, TileCfg<D, V>::kMinBl
             self = sm.coff[own] + (s - sm.cglob[own]);
             if (DBG) acc.cand += j1 - j0 - 1;
         }
+        // The lanes of a cell read the same candidates; the r-th cell of the
+        // warp starts up to 7 before its window, at a staged index of r mod 8,
+        // so that the cells' 16-byte loads fall into different banks
+        // (250k uniform particles 87.1 -> 85.6 us, 4M blobs 1157 -> 1148 us).
+        const int js = j0 - ((j0 - __popc(leads & (kFull >> (31 - lane)))) & 7);
         const LoopK K(P);
         const float neg_thr = -(float)P.rmax2 * (1.f + kCullRel);
         float umin = INFINITY;
@@ -481,7 +488,7 @@ __global__ void __launch_bounds__(TileCfg<D, V>::kTargets, TileCfg<D, V>::kMinBl
         auto walk = [&](auto shifted) {
             constexpr bool kShifted = decltype(shifted)::value;
             const float px1 = px - 1.f, py1 = py - 1.f, pz1 = pz - 1.f;
-            for (int j = j0; j < j1; j += 32 * kCullWords) {
+            for (int j = js; j < j1; j += 32 * kCullWords) {
                 const int nw = min(kCullWords, (j1 - j + 31) >> 5);
                 // The words that keep something, with the staged index of
                 // their bit 31, and how many candidates they keep.
@@ -490,6 +497,7 @@ __global__ void __launch_bounds__(TileCfg<D, V>::kTargets, TileCfg<D, V>::kMinBl
                 for (int i = 0; i < nw; ++i) {
                     const int base = j + 32 * i;
                     uint32_t m = cull_word<kShifted>(sm.cand + base, min(32, j1 - base), px, py, pz, neg_thr);
+                    if (base < j0) m &= kFull >> (j0 - base);
                     if ((unsigned)(self - base) < 32u) m &= ~(0x80000000u >> (self - base));
                     if (m) {
                         *put = make_uint2(m, (uint32_t)base + 31);
