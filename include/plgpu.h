@@ -302,9 +302,10 @@ int plg_set_use_graph(plg_ctx* ctx, int32_t on);
 
 /* Force kernel tile variant of this world (see PLG_TILE_VARIANTS below).
  * Until plg_set_tile or plg_autotune chooses one, 2D worlds under 300,000
- * particles use variant 2 and all others variant 0, except crowded 2D worlds
- * (48 particles per cell or more on average): variant 1.  Every variant gives
- * the same bits. */
+ * particles use variant 2 and larger ones variant 0, except crowded 2D worlds
+ * (48 particles per cell or more on average): variant 1.  3D worlds use
+ * variant 0, from 200,000 particles on with fewer than 11 per cell variant 2.
+ * Every variant gives the same bits. */
 int plg_set_tile(plg_ctx* ctx, int32_t variant);
 int plg_get_tile(plg_ctx* ctx, int32_t* variant);
 /* Times `steps` steps of every tile variant on the world as it is
@@ -428,7 +429,7 @@ int plg_batch_step_stats(plg_batch* batch, int64_t* deferred);
 /* Force kernel tile variants (threads = targets per block, staging size):
  * 2D: 0 = 128 targets / 1152 staged candidates, 1 = 128 / 2048 (crowded
  * worlds), 2 = 128 / 1280 with more registers (small worlds); 3D: 0 = 128 /
- * 2176, 1 = 64 / 832 (sparse worlds), 2 = 128 / 1728 (more blocks per SM).
+ * 2176, 1 = 64 / 832 (sparse worlds), 2 = 128 / 1776 (large worlds).
  * All give the same bits.  Until a variant is set or tuned, a world joins
  * with variant 0, or 1 when it is a crowded 2D world (plg_set_tile).  Each world
  * of a batch has its own variant; a step launches the force kernel once per

@@ -145,13 +145,15 @@ __global__ void __launch_bounds__(kThreads) k_force_general(const __grid_constan
 // 1: 2048 candidates at 6 blocks for crowded cells (400k particles, 119 per
 // cell: 330 us against 498, 60 per cell: 169 against 172).  Variant 2: 7
 // blocks with more registers and candidates, for worlds of about one wave.
-// 3D: variant 0 (4 blocks of 128 targets) holds 71 staged columns of 9 cells,
-// so that the sparse tails of a blob world stage in one or two rounds, and
-// 2176 candidates for the dense cores; variant 1 is the smaller tile for
-// sparse worlds.
-// 3D variant 2: 5 blocks of 128
-// targets with 1728 candidates (4M blobs: force 1157 us against 1169 for
-// variant 0; 1M uniform with 50 neighbours: 359 against 323).
+// 3D: 71 staged columns of 9 cells in variants 0 and 2, so that the sparse
+// tails of a blob world stage in one or two rounds.  Variant 0: 4 blocks of
+// 128 targets with 2176 candidates, for dense cells and for worlds of about
+// one wave.  Variant 1: the smaller tile for small sparse worlds.  Variant 2:
+// 5 blocks of 128 targets with 1776 candidates, as much shared memory as five
+// blocks have, for large worlds (4M in blobs 1066 us against variant 0's 1148;
+// with 448 cells it took 1108, with 832 cells and 1600 candidates 1124; 1M at
+// 2.5 per cell 135 us against 147, 163 with 448 cells; six blocks of 1216
+// candidates 165).
 template <int D, int V>
 struct TileCfg;
 template <>
@@ -176,13 +178,14 @@ struct TileCfg<3, 1> {
 };
 template <>
 struct TileCfg<3, 2> {
-    static constexpr int kTargets = 128, kMinBlocks = 5, kCap = 1728, kCells = 448;
+    static constexpr int kTargets = 128, kMinBlocks = 5, kCap = 1776, kCells = 640;
 };
 
 // Words of 32 candidates a 3D target tests before it forms the kept terms.
 constexpr int kCullWords = 8;
 
-// Lives in dynamic shared memory (variant 0: about 28 KB in 2D, 42 KB in 3D).
+// Lives in dynamic shared memory (22 KB in 2D variant 0; 51 KB in 3D
+// variant 0, 44 KB in variant 2).
 // Staged columns: the sorted union of the windows cx-1..cx+1 of the staged
 // targets, as "virtual" columns -1..nx (-1 and nx being the periodic images
 // of columns nx-1 and 0), each with the grid row of its segment.

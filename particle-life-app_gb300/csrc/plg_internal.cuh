@@ -413,6 +413,17 @@ int tile_targets(int dim, int variant);
 constexpr int64_t kCrowdedCell2D = 48;
 inline bool crowded_world(int dim, int64_t n, int64_t ncells) { return dim == 2 && n >= kCrowdedCell2D * ncells; }
 
+// A 3D world below this many particles per cell on average is better off with
+// five blocks per SM (variant 2) than with variant 0's longer staging of
+// denser cells, once it fills the machine (kFullWorld3D): 1M particles, force
+// kernel, variant 0 -> 2: 2.4 per cell 147 -> 135 us, 6.0 per cell 188 -> 173,
+// 10.3 per cell 268 -> 255, 12.6 per cell 316 -> 320, 27.8 per cell 718 -> 812;
+// 4M in blobs, 0.3 per cell, 1148 -> 1066.  A world that clusters further
+// keeps the gain (the mean does not see it): 1M in blobs of 0.03 with 40
+// neighbours 308 -> 288.
+constexpr int64_t kDenseCell3D = 11;
+inline bool open_world(int dim, int64_t n, int64_t ncells) { return dim == 3 && n < kDenseCell3D * ncells; }
+
 // Opts the tiled force kernel in to its dynamic shared memory (> 48 KB) on
 // the current device; called once per context.
 cudaError_t force_kernels_init();

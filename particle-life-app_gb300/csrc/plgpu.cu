@@ -313,11 +313,17 @@ Grid grid_of(plg_ctx* c) { return c->fp.g; }
 // at most two waves of blocks, and its extra registers count for more than
 // variant 0's eighth block.
 constexpr int64_t kSmallWorld2D = 300000;
+// 3D worlds of this many particles run more than two waves of blocks, where
+// variant 2's fifth block per SM counts (250k particles at 2.4 per cell 49 ->
+// 44 us, at 9.3 per cell 82 -> 82); at one wave it only lengthens the wave
+// (120k at 2.6 per cell: 30 -> 36 us).
+constexpr int64_t kFullWorld3D = 200000;
 
 // The tile variant a step uses: the one set or tuned, else by size.
 int tile_variant(const plg_ctx* c) {
     if (!c->variant_auto) return c->variant;
     if (crowded_world(c->dim, c->n, c->ncells)) return 1;
+    if (c->n >= kFullWorld3D && open_world(c->dim, c->n, c->ncells)) return 2;
     return c->dim == 2 && c->n < kSmallWorld2D ? 2 : 0;
 }
 
