@@ -275,12 +275,14 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const uint32_t* __restric
                                                        uint32_t* __restrict__ cstart, unsigned long long* state,
                                                        uint32_t* status, uint32_t* zero_word) {
     __shared__ uint32_t s_tile, s_prefix, total;
-    pdl_release();  // the scatter's blocks may be scheduled as this grid ends
     if (threadIdx.x == 0) s_tile = atomicAdd(reinterpret_cast<unsigned int*>(state), 1u);
     // Launched after the force kernel (launch_scan's `after`), the blocks
     // may start while it drains: the counts and the deferred-target count
     // are read or reset only once it has completed.
     pdl_wait();
+    // The scatter's blocks may be scheduled as this grid ends, but not while
+    // the force kernel still runs: they would wait on the SMs it needs.
+    pdl_release();
     __syncthreads();
     const int tile = (int)s_tile;
     if (tile == 0 && threadIdx.x == 0 && zero_word) *zero_word = 0u;  // the step's deferred-target count
@@ -381,13 +383,16 @@ __global__ void __launch_bounds__(kThreads) k_scatter(int n, const uint32_t* __r
     uint32_t c[kScatterPer], top[kScatterPer];
     unsigned peers[kScatterPer];
     bool v[kScatterPer];
+    // The scan's offsets, and its reads of the counts, are done.  The cells
+    // too are read only now: they come from the force kernel, which the scan
+    // has waited for, and this grid may have been scheduled before that.
+    pdl_wait();
 #pragma unroll
     for (int k = 0; k < kScatterPer; ++k) {
         const int i = i0 + k * kThreads;
         v[k] = i < n;
-        c[k] = v[k] ? cell[i] : 0u;  // written before the scan: needs no wait
+        c[k] = v[k] ? cell[i] : 0u;
     }
-    pdl_wait();  // the scan's offsets, and its reads of the counts, are done
     if (zero_state && blockIdx.x == 0)
         for (int k = threadIdx.x; k < nzero; k += kThreads) zero_state[k] = 0ull;
 #pragma unroll
