@@ -36,7 +36,7 @@ struct ForceArgs {
     const ForceParams* __restrict__ worlds;
     const int* __restrict__ wp_off;
     const int* __restrict__ tile_off;
-    const int* __restrict__ steps_left;  // per world; <= 0: frozen this step (may be null)
+    const int* __restrict__ steps_left;  // per world; < 0: frozen this step (may be null)
     unsigned long long* wcycles;         // per world: SM cycles of its blocks (autotuner; may be null)
     int nworlds;
     int n_total;

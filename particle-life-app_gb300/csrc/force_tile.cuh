@@ -10,8 +10,8 @@
 // and, in its epilogue, the counting pass of the next makeContainers
 // (Physics.java:328-332) on the new position.
 //
-// Tiling.  A block takes 128 consecutive targets of the sorted order (tile
-// variant 0), one thread each; their cells come from the sort.  The cells are
+// Tiling.  A block takes 128 (3D variant 1: 64) consecutive targets of the
+// sorted order, one thread each; their cells come from the sort.  The cells are
 // nondecreasing, so the targets fall into a few "segments" (targets of one
 // grid row: one y in 2D, one (y, z) in 3D).  A target in column cx needs the
 // window of columns cx-1..cx+1 over its R stencil rows (3 in 2D, 9 in 3D);
@@ -306,7 +306,7 @@ __device__ __forceinline__ bool stage_columns(const ForceArgs<D>& A, const Force
 }
 
 // Main force kernel (nx >= 3): one thread per target; a block takes
-// kTargets (128 in variant 0) consecutive targets and stages their windows
+// kTargets consecutive targets and stages their windows
 // so that each target reads one contiguous run (or, where a window does not
 // fit, reads the same cells from global memory).  Neighbouring threads mostly share a cell, hence a
 // window, so their candidate loads are broadcasts.  FP32 only: a target
@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(TileCfg<D, V>::kTargets, TileCfg<D, V>::kMinBl
     const bool valid = tid < nvalid;
     const int s = s0 + tid;
     const ForceParams& P = BATCH ? A.worlds[wk] : A.p;
-    if (BATCH && A.steps_left && __ldg(A.steps_left + wk) <= 0) {
+    if (BATCH && A.steps_left && __ldg(A.steps_left + wk) < 0) {
         // A world that has used up its steps is left exactly as its last
         // step left it: A (its state, in that step's order) is not touched,
         // and the cells that step computed for it are counted again for the

@@ -162,11 +162,6 @@ __global__ void __launch_bounds__(kThreads) k_batch_rebin(int n, StateBuf<D> a, 
     }
 }
 
-__global__ void k_batch_tick(int* steps_left, int nworlds) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < nworlds && steps_left[k] > 0) steps_left[k] -= 1;
-}
-
 // Re-binning of the current state (after an rmax change, or of a world
 // generated on the device; cell_base: the world's first global cell).
 template <int D>
@@ -376,7 +371,8 @@ constexpr int kScatterPer = 4;
 __global__ void __launch_bounds__(kThreads) k_scatter(int n, const uint32_t* __restrict__ cell, uint32_t* counts,
                                                       const uint32_t* __restrict__ cstart,
                                                       uint32_t* __restrict__ perm, uint32_t* __restrict__ slot_cell,
-                                                      unsigned long long* zero_state, int nzero) {
+                                                      unsigned long long* zero_state, int nzero, int* steps_left,
+                                                      int nworlds) {
     pdl_release();
     const int i0 = blockIdx.x * (kThreads * kScatterPer) + threadIdx.x;
     const int lane = threadIdx.x & 31;
@@ -395,6 +391,10 @@ __global__ void __launch_bounds__(kThreads) k_scatter(int n, const uint32_t* __r
     }
     if (zero_state && blockIdx.x == 0)
         for (int k = threadIdx.x; k < nzero; k += kThreads) zero_state[k] = 0ull;
+    // Batched worlds: this step off each world's budget (the force kernels
+    // of the step before have completed, this step's start after this grid).
+    if (steps_left && blockIdx.x == gridDim.x - 1)
+        for (int k = threadIdx.x; k < nworlds; k += kThreads) steps_left[k] = max(steps_left[k], 0) - 1;
 #pragma unroll
     for (int k = 0; k < kScatterPer; ++k) {
         const unsigned m = __ballot_sync(kFull, v[k]);
@@ -594,11 +594,6 @@ void launch_batch_rebin(cudaStream_t st, int n, StateBuf<D> a, const ForceParams
     k_batch_rebin<D><<<blocks_for(n, kThreads), kThreads, 0, st>>>(n, a, worlds, wp_off, nw, cell, counts);
 }
 
-void launch_batch_tick(cudaStream_t st, int* steps_left, int nworlds) {
-    if (nworlds <= 0 || !steps_left) return;
-    k_batch_tick<<<blocks_for(nworlds, kThreads), kThreads, 0, st>>>(steps_left, nworlds);
-}
-
 template void launch_batch_move<2>(cudaStream_t, int, const int*, const int*, int, StateBuf<2>, StateBuf<2>);
 template void launch_batch_move<3>(cudaStream_t, int, const int*, const int*, int, StateBuf<3>, StateBuf<3>);
 template void launch_batch_rebin<2>(cudaStream_t, int, StateBuf<2>, const ForceParams*, const int*, int, uint32_t*,
@@ -632,10 +627,11 @@ void launch_scan(cudaStream_t st, const uint32_t* counts, int ncells, uint32_t* 
 }
 
 void launch_scatter(cudaStream_t st, int n, const uint32_t* cell, uint32_t* counts, const uint32_t* cstart,
-                    uint32_t* perm, uint32_t* slot_cell, unsigned long long* zero_state, int nzero) {
+                    uint32_t* perm, uint32_t* slot_cell, unsigned long long* zero_state, int nzero, int* steps_left,
+                    int nworlds) {
     if (n <= 0) return;
     launch_after(k_scatter, dim3(blocks_for(n, kThreads * kScatterPer)), dim3(kThreads), 0, st, n, cell, counts,
-                 cstart, perm, slot_cell, zero_state, nzero);
+                 cstart, perm, slot_cell, zero_state, nzero, steps_left, nworlds);
 }
 
 bool sort_is_small(int n, int ncells) { return n > 0 && n <= kSmallParticles && ncells <= kSmallCells; }

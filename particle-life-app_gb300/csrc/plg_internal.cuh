@@ -337,10 +337,12 @@ void launch_scan(cudaStream_t st, const uint32_t* counts, int ncells, uint32_t* 
 // slot_cell (may be null): receives the cell of each sorted slot.
 // zero_state (may be null): nzero words the scan before it used (its tile
 // counter and look-back flags), set back to zero for the next step's scan.
+// steps_left (may be null): the step budgets of nworlds batched worlds; each
+// is counted down by one, to -1 where none was left.
 // A programmatic dependent of the scan (launch_after).
 void launch_scatter(cudaStream_t st, int n, const uint32_t* cell, uint32_t* counts, const uint32_t* cstart,
                     uint32_t* perm, uint32_t* slot_cell = nullptr, unsigned long long* zero_state = nullptr,
-                    int nzero = 0);
+                    int nzero = 0, int* steps_left = nullptr, int nworlds = 0);
 
 template <int D>
 void launch_gather(cudaStream_t st, int n, const uint32_t* perm, const uint32_t* slot_cell, const uint32_t* cstart,
@@ -365,7 +367,7 @@ void launch_sort_small(cudaStream_t st, int n, int ncells, const uint32_t* cell,
 // slot_cell: the cell of each slot of b, as the scatter wrote it.
 // `defer`: one word, zeroed before the step; counts the targets the tiled
 // kernel recomputed in its deferred pass.
-// variant: tile variant of the force kernel (0 or 1, the autotuner's knob).
+// variant: tile variant of the force kernel (0 .. PLG_TILE_VARIANTS - 1).
 // snap (tiled kernel only, not with dbg; may be null): also write the new
 // state to these arrays (see HostSnap).
 template <int D>
@@ -379,7 +381,7 @@ void launch_force(cudaStream_t st, const ForceParams& p, bool general, StateBuf<
 // nworlds + 1) the first tile of each world for this variant's tile size
 // (tile_targets), `tiles` the total.  Every world has nx >= 3.
 // smem_matrix: every world has at most 16 types.
-// steps_left (device, per world, may be null): a world at <= 0 is frozen
+// steps_left (device, per world, may be null): a world at < 0 is frozen
 // for the step (its state and order untouched, its cells counted again).
 // wcycles (device, per world, may be null): each block adds its duration in
 // SM cycles to its world's entry (the per-world autotuner).
@@ -393,8 +395,6 @@ void launch_force_batch(cudaStream_t st, const ForceParams* worlds, const int* w
 // Resident blocks per SM of the batched force kernel of a tile variant.
 int batch_blocks_per_sm(int dim, int variant, bool smem_matrix);
 
-// Counts every positive steps_left[k] (k < nworlds) down by one.
-void launch_batch_tick(cudaStream_t st, int* steps_left, int nworlds);
 
 // The autotuners' choice: the fastest variant `best` replaces the current
 // one only when it is at least 2% faster, so timing noise between nearly
