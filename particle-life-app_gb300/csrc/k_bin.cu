@@ -28,10 +28,13 @@ constexpr int kScanThreads = 256;
 constexpr int kScanItems = 16;
 constexpr int kScanTile = kScanThreads * kScanItems;
 
-// k_sort_small: threads per block, slots a block is given (at most
-// kSmallBlocks blocks) and members its shared list holds.
-constexpr int kSmallThreads = 1024, kSmallShare = 512, kSmallBlocks = 128;
-constexpr uint32_t kSmallList = 4096;
+// k_sort_small: threads per block, slots of a block's share (at most), and the
+// most members of a cell that is not crowded (a share meets at most
+// kSmallCrowds of the others).
+constexpr int kSmallThreads = 1024, kSmallShare = 512, kSmallCrowd = 512;
+constexpr int kSmallCrowds = kSmallShare / kSmallCrowd + 2, kSmallList = kSmallShare + kSmallCrowd;
+constexpr uint32_t kNoMember = ~0u;
+static_assert(kSmallList <= kSmallThreads, "a thread per list entry");
 
 inline int blocks_for(int n, int threads) { return (n + threads - 1) / threads; }
 
@@ -451,44 +454,57 @@ __global__ void __launch_bounds__(kThreads) k_gather(int n, const uint32_t* __re
 // k_scan, k_scatter and k_gather of a small world (sort_is_small) without
 // any exchange between blocks: every block counts all the cells from the
 // particles' cell indices in its own shared memory and scans them, then
-// sorts the cells whose first slot falls into its share of the slots.  A
-// small world's three launches are a chain of memory and launch latencies,
-// 3 to 4 us each however little they move; re-reading 4 bytes per particle
-// in every block costs less than handing results from block to block.
+// sorts its share of the slots.  A small world's three launches are a chain
+// of memory and launch latencies, 3 to 4 us each however little they move;
+// re-reading 4 bytes per particle in every block costs less than handing
+// results from block to block.
+// A cell belongs to the block whose share it starts in, which ranks its
+// members against one another, m^2 compares for m members.  A crowded cell
+// (more than kSmallCrowd) is not ranked: every block whose share it meets
+// walks all the cell indices in order once and moves the members that fall
+// into its share, so that the work is n per block and spread over the blocks
+// however large the cell.  (Ranked by one block like the others, 24,576
+// particles in one cell took 21.5 ms to sort, in 9 cells 219 us, in 25 64;
+// now 22, 26 and 25, against 565, 90 and 44 in the three launches.  The line
+// at 512 members: with 256, 100 cells of 246 took 28 us instead of 19.)
 template <int D>
 __global__ void __launch_bounds__(kSmallThreads) k_sort_small(int n, int ncells, const uint32_t* __restrict__ cell,
                                                               uint32_t* __restrict__ counts,
-                                                              uint32_t* __restrict__ cstart, uint32_t* perm,
+                                                              uint32_t* __restrict__ cstart,
                                                               uint32_t* __restrict__ slot_cell, StateBuf<D> a,
                                                               StateBuf<D> b, int32_t* __restrict__ cell_sorted,
                                                               uint32_t* zero_word) {
     extern __shared__ uint32_t small_smem[];
     uint32_t* const start = small_smem;              // first slot of each cell, ncells + 1
     uint32_t* const next = start + ncells + 1;       // next free slot of each cell
-    uint32_t* const list = next + ncells;            // members of this block's slots
-    __shared__ uint32_t warp_sum[kSmallThreads / 32], own[2];
+    uint32_t* const list = next + ncells;            // members of the block's cells, by slot - lo
+    __shared__ uint32_t warp_sum[2][kSmallThreads / 32], crowd[kSmallCrowds], ncrowd;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int all = blockIdx.x * kSmallThreads + tid, nall = gridDim.x * kSmallThreads;
     for (int c = tid; c < ncells; c += kSmallThreads) start[c] = 0u;
-    if (tid < 2) own[tid] = 0u;
+    if (tid < kSmallList) list[tid] = kNoMember;
+    if (tid == 0) ncrowd = 0u;
     __syncthreads();
     pdl_wait();  // the force kernel's cells
     if (zero_word && all == 0) *zero_word = 0u;  // the step's deferred-target count
     for (int c = all; c < ncells; c += nall) counts[c] = 0u;  // for the next counting pass
     // Four consecutive particles per thread: of one or two cells in a world
     // that has been sorted before, so they count once or twice.
+    auto load4 = [&](int i, int m) {
+        uint4 q = make_uint4(0u, 0u, 0u, 0u);
+        if (m == 4) {
+            q = *reinterpret_cast<const uint4*>(cell + i);
+        } else {
+            if (m > 0) q.x = cell[i];
+            if (m > 1) q.y = cell[i + 1];
+            if (m > 2) q.z = cell[i + 2];
+        }
+        return q;
+    };
     auto each4 = [&](auto f) {
         for (int i = 4 * tid; i < n; i += 4 * kSmallThreads) {
-            uint4 q = make_uint4(0u, 0u, 0u, 0u);
             const int m = min(4, n - i);
-            if (m == 4) {
-                q = *reinterpret_cast<const uint4*>(cell + i);
-            } else {
-                q.x = cell[i];
-                if (m > 1) q.y = cell[i + 1];
-                if (m > 2) q.z = cell[i + 2];
-            }
-            f(i, m, q);
+            f(i, m, load4(i, m));
         }
     };
     each4([&](int, int m, uint4 q) {
@@ -509,40 +525,43 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(int n, int ncells,
     });
     __syncthreads();
     // Exclusive scan of the counts in place, an odd number of cells per
-    // thread (no bank conflicts); the cell holding a boundary of this block's
-    // share of the slots tells where its own slots begin and end.
+    // thread (no bank conflicts), noting the crowded cells of this block's
+    // share [lo, hi) of the slots.
     const int per = ((ncells + kSmallThreads - 1) / kSmallThreads) | 1;
     const int c0 = min(tid * per, ncells), c1 = min(c0 + per, ncells);
     uint32_t sum = 0;
     for (int c = c0; c < c1; ++c) sum += start[c];
     const uint32_t inc = warp_inclusive(sum);
-    if (lane == 31) warp_sum[warp] = inc;
+    if (lane == 31) warp_sum[0][warp] = inc;
     __syncthreads();
     if (warp == 0) {
-        const uint32_t s = warp_sum[lane];
-        warp_sum[lane] = warp_inclusive(s) - s;
+        const uint32_t s = warp_sum[0][lane];
+        warp_sum[0][lane] = warp_inclusive(s) - s;
     }
     __syncthreads();
     const uint32_t lo = (uint32_t)((int64_t)n * blockIdx.x / gridDim.x);
     const uint32_t hi = (uint32_t)((int64_t)n * (blockIdx.x + 1) / gridDim.x);
-    uint32_t run = warp_sum[warp] + inc - sum;
+    uint32_t run = warp_sum[0][warp] + inc - sum;
     for (int c = c0; c < c1; ++c) {
         const uint32_t end = run + start[c];
+        if (end - run > kSmallCrowd && run < hi && end > lo) crowd[atomicAdd(&ncrowd, 1u)] = (uint32_t)c;
         start[c] = run;
         next[c] = run;
-        if (run < lo && lo <= end) own[0] = end;
-        if (run < hi && hi <= end) own[1] = end;
         run = end;
     }
     if (tid == 0) start[ncells] = (uint32_t)n;
     __syncthreads();
-    const uint32_t own0 = own[0], own1 = own[1];
-    // The members of the block's cells, in any order within a cell; where
-    // they exceed the shared list, in the block's slots of perm.
-    uint32_t* const mem = own1 - own0 <= kSmallList ? list - own0 : perm;
+    auto move = [&](uint32_t i, uint32_t slot, uint32_t c) {
+        slot_cell[slot] = c;
+        b.pt[slot] = a.pt[i];
+        b.vel[slot] = a.vel[i];
+        if (cell_sorted) cell_sorted[slot] = (int32_t)c;
+    };
+    // The members of the block's cells, in any order within a cell.
     each4([&](int i, int m, uint4 q) {
         auto take = [&](int k, uint32_t c) {
-            if (k < m && start[c] >= lo && start[c] < hi) mem[atomicAdd(next + c, 1u)] = (uint32_t)(i + k);
+            if (k < m && start[c] >= lo && start[c] < hi && start[c + 1] - start[c] <= kSmallCrowd)
+                list[atomicAdd(next + c, 1u) - lo] = (uint32_t)(i + k);
         };
         take(0, q.x);
         take(1, q.y);
@@ -551,17 +570,37 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(int n, int ncells,
     });
     __syncthreads();
     // Stable order within the cell: the members of a smaller index go first.
-    for (uint32_t s = own0 + tid; s < own1; s += kSmallThreads) {
-        const uint32_t i = mem[s], c = cell[i];
-        const float4 p = a.pt[i];
-        const typename Layout<D>::Vel v = a.vel[i];
-        const uint32_t st = start[c], en = start[c + 1];
+    if (tid < kSmallList && list[tid] != kNoMember) {
+        const uint32_t i = list[tid], c = cell[i], st = start[c], en = start[c + 1];
         uint32_t r = 0;
-        for (uint32_t t = st; t < en; ++t) r += mem[t] < i ? 1u : 0u;
-        slot_cell[s] = c;
-        b.pt[st + r] = p;
-        b.vel[st + r] = v;
-        if (cell_sorted) cell_sorted[st + r] = (int32_t)c;
+        for (uint32_t t = st - lo; t < en - lo; ++t) r += list[t] < i ? 1u : 0u;
+        move(i, st + r, c);
+    }
+    // Crowded cells: their members in the order of the walk, those of this
+    // block's slots moved.
+    int turn = 0;  // of the two rows of warp sums
+    for (uint32_t q = 0; q < ncrowd; ++q) {
+        const uint32_t c = crowd[q];
+        uint32_t first = start[c];  // slot of the next member
+        for (int i0 = 0; i0 < n && first < hi; i0 += 4 * kSmallThreads, turn ^= 1) {
+            const int i = i0 + 4 * tid, m = max(0, min(4, n - i));
+            const uint4 v = load4(i, m);
+            const bool is[4] = {m > 0 && v.x == c, m > 1 && v.y == c, m > 2 && v.z == c, m > 3 && v.w == c};
+            const uint32_t mine = (uint32_t)is[0] + is[1] + is[2] + is[3];
+            const uint32_t upto = warp_inclusive(mine);
+            if (lane == 31) warp_sum[turn][warp] = upto;
+            __syncthreads();
+            const uint32_t w = warp_inclusive(warp_sum[turn][lane]);
+            const uint32_t before = __shfl_sync(kFull, w, max(warp - 1, 0));
+            uint32_t slot = first + (warp > 0 ? before : 0u) + upto - mine;
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (is[k]) {
+                    if (slot >= lo && slot < hi) move((uint32_t)(i + k), slot, c);
+                    ++slot;
+                }
+            first += __shfl_sync(kFull, w, 31);
+        }
     }
     for (int c = all; c <= ncells; c += nall) cstart[c] = start[c];
 }
@@ -642,15 +681,15 @@ size_t small_sort_smem(int ncells) { return sizeof(uint32_t) * (2 * (size_t)ncel
 
 template <int D>
 void launch_sort_small(cudaStream_t st, int n, int ncells, const uint32_t* cell, uint32_t* counts, uint32_t* cstart,
-                       uint32_t* perm, uint32_t* slot_cell, StateBuf<D> a, StateBuf<D> b, int32_t* cell_sorted,
-                       uint32_t* zero_word, bool after) {
-    const dim3 grid(std::min(kSmallBlocks, blocks_for(n, kSmallShare))), block(kSmallThreads);
+                       uint32_t* slot_cell, StateBuf<D> a, StateBuf<D> b, int32_t* cell_sorted, uint32_t* zero_word,
+                       bool after) {
+    const dim3 grid(blocks_for(n, kSmallShare)), block(kSmallThreads);
     const size_t smem = small_sort_smem(ncells);
     if (after)
-        launch_after(k_sort_small<D>, grid, block, smem, st, n, ncells, cell, counts, cstart, perm, slot_cell, a, b,
+        launch_after(k_sort_small<D>, grid, block, smem, st, n, ncells, cell, counts, cstart, slot_cell, a, b,
                      cell_sorted, zero_word);
     else
-        k_sort_small<D><<<grid, block, smem, st>>>(n, ncells, cell, counts, cstart, perm, slot_cell, a, b, cell_sorted,
+        k_sort_small<D><<<grid, block, smem, st>>>(n, ncells, cell, counts, cstart, slot_cell, a, b, cell_sorted,
                                                    zero_word);
 }
 
@@ -661,9 +700,9 @@ cudaError_t sort_kernels_init() {
     return cudaFuncSetAttribute(k_sort_small<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
-template void launch_sort_small<2>(cudaStream_t, int, int, const uint32_t*, uint32_t*, uint32_t*, uint32_t*, uint32_t*,
+template void launch_sort_small<2>(cudaStream_t, int, int, const uint32_t*, uint32_t*, uint32_t*, uint32_t*,
                                    StateBuf<2>, StateBuf<2>, int32_t*, uint32_t*, bool);
-template void launch_sort_small<3>(cudaStream_t, int, int, const uint32_t*, uint32_t*, uint32_t*, uint32_t*, uint32_t*,
+template void launch_sort_small<3>(cudaStream_t, int, int, const uint32_t*, uint32_t*, uint32_t*, uint32_t*,
                                    StateBuf<3>, StateBuf<3>, int32_t*, uint32_t*, bool);
 
 template <int D>

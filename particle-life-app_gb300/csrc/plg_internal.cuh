@@ -349,8 +349,8 @@ void launch_gather(cudaStream_t st, int n, const uint32_t* perm, const uint32_t*
                    StateBuf<D> a, StateBuf<D> b, int32_t* cell_sorted);
 
 // The three launches above as one, for small worlds (sort_is_small): the
-// same cstart, slot_cell and B; the counts are set to zero (not read), and
-// perm is scratch.  after: a programmatic dependent of the kernel before it.
+// same cstart, slot_cell and B; the counts are set to zero (not read).
+// after: a programmatic dependent of the kernel before it.
 // sort_kernels_init: once per context.
 // The line: every block reads all n cells, so the single launch wins while
 // that is cheaper than two more launches (2D steps with it and without: 1,000
@@ -361,8 +361,8 @@ bool sort_is_small(int n, int ncells);
 cudaError_t sort_kernels_init();
 template <int D>
 void launch_sort_small(cudaStream_t st, int n, int ncells, const uint32_t* cell, uint32_t* counts, uint32_t* cstart,
-                       uint32_t* perm, uint32_t* slot_cell, StateBuf<D> a, StateBuf<D> b, int32_t* cell_sorted,
-                       uint32_t* zero_word, bool after);
+                       uint32_t* slot_cell, StateBuf<D> a, StateBuf<D> b, int32_t* cell_sorted, uint32_t* zero_word,
+                       bool after);
 
 // slot_cell: the cell of each slot of b, as the scatter wrote it.
 // `defer`: one word, zeroed before the step; counts the targets the tiled

@@ -347,8 +347,8 @@ void enqueue_body(plg_ctx* c, const DebugOut* dbg, int32_t* cell_sorted, const H
     const bool small = sort_is_small(n, c->ncells);
     k0(PLG_K_SCAN);
     if (small)  // the whole sort (profiled as the scan)
-        launch_sort_small<D>(st, n, c->ncells, c->cell, c->counts, c->cstart, c->perm, c->slot_cell, buf_a<D>(c),
-                             buf_b<D>(c), cell_sorted, zero_word, !c->profiling);
+        launch_sort_small<D>(st, n, c->ncells, c->cell, c->counts, c->cstart, c->slot_cell, buf_a<D>(c), buf_b<D>(c),
+                             cell_sorted, zero_word, !c->profiling);
     else
         launch_scan(st, c->counts, c->ncells, c->cstart, c->scan_state, c->status_d, zero_word, !c->profiling);
     k1(PLG_K_SCAN);
