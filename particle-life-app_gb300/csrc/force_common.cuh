@@ -522,7 +522,8 @@ __device__ __forceinline__ int staged_global(const int* coff, const int* cglob, 
 }
 
 // 2D: the staged candidates [j0, j1) of a target, itself at self_j among the
-// members [o0, o1) of its own cell, from a column-major staging (cand, with
+// members [o0, o1) of its own cell (a part of the window without that cell:
+// o0 = o1 = j1, self_j < 0), from a column-major staging (cand, with
 // cell offsets coff and global starts cglob of ncell cells).  Branch-free
 // FP32: every lane evaluates the Accelerator for every candidate, and a pair
 // beyond rmax adds an exact zero (cand_term).  The target's own copy is moved
@@ -650,8 +651,8 @@ __device__ __forceinline__ uint32_t cull_word(const float4* __restrict__ cand, i
     return n < 32 ? m & ~(kFull >> n) : m;
 }
 
-// The target's neighbourhood read straight from global memory, for segments
-// too wide or too full for shared memory: the cells in the staged order
+// The target's neighbourhood read straight from global memory, for windows
+// with a cell too full for shared memory: the cells in the staged order
 // (columns cx-1..cx+1, and in each the R stencil rows), the same image
 // shifts (below the box: the candidate's coordinate minus 1; above: the
 // target's) and the same candidate evaluation, so the sum has the same bits

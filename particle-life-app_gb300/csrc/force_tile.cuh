@@ -19,10 +19,11 @@
 // memory column by column, each column's R cells in turn, so that every
 // target's neighbourhood is one contiguous run.  When the whole block's
 // windows fit, one staging serves every target; otherwise the block's
-// columns are staged in chunks (which may span segments), halved until they
-// fit, and a single window that still does not fit (a very dense region) is
-// read from global memory in the same candidate order (direct_stencil),
-// giving the same bits.  The 2D
+// cells are staged in parts, as many at a time as fit, and each part serves
+// every target whose window meets it.  A cell that does not fit by itself
+// (a very dense region) sends the targets that need it to global memory
+// (direct_stencil).  The candidates come in the same order and give the same
+// bits throughout.  The 2D
 // candidate loop is branch-free FP32; a 3D window is tested by distance
 // first, and terms are formed for what that keeps.  A target that meets a
 // candidate needing the FP64 decision is deferred: its warp recomputes it from global
@@ -186,7 +187,7 @@ constexpr int kCullWords = 8;
 
 // Lives in dynamic shared memory (22 KB in 2D variant 0; 51 KB in 3D
 // variant 0, 44 KB in variant 2).
-// Staged columns: the sorted union of the windows cx-1..cx+1 of the staged
+// Listed columns: the sorted union of the windows cx-1..cx+1 of the staged
 // targets, as "virtual" columns -1..nx (-1 and nx being the periodic images
 // of columns nx-1 and 0), each with the grid row of its segment.
 template <int D, int V>
@@ -207,10 +208,10 @@ struct TileSmem {
     uint8_t image[TileCfg<D, V>::kCells];  // image shifts of stencil cell e (kUp*, kDown*)
 };
 
-// Stages the cells of staged columns 0..ncols-1 (sm.colv, sm.colrow),
-// column-major: for each column the cells of its R stencil rows in turn, so
-// that the neighbourhood of a target whose window starts at column k is the
-// single contiguous range of columns k .. k+2.  Images below the box are
+// Stages ncell cells of the listed columns (sm.colv, sm.colrow), from cell
+// `off` of the first one on, column-major: for each column the cells of its R
+// stencil rows in turn, so that the neighbourhood of a target whose window
+// starts at column k is the single contiguous range of columns k .. k+2.  Images below the box are
 // shifted down by 1 here (exact: their coordinates are >= 0.5); images above
 // it are flagged for a target shift instead.  Thread t places cells
 // t*per .. t*per+per-1: it reads their extents, and the block scans the
@@ -221,17 +222,17 @@ struct TileSmem {
 // staging and the target rows without integer divisions, together: force
 // kernel of 1M particles in 2D 95.9 -> 88.3 us, of 4M in 3D blobs 1383 ->
 // 1187 us.)
-// Returns whether the candidates fit (every thread gets the same answer);
-// ncols * R <= kCells is the caller's.
+// Returns the number of cells staged (the same in every thread): as many of
+// the first ones as fit, 0 when not even one does; ncell <= kCells is the
+// caller's.
 template <int D, int V>
-__device__ __forceinline__ bool stage_columns(const ForceArgs<D>& A, const ForceParams& P,
-                                              const uint32_t* __restrict__ cs, TileSmem<D, V>& sm, int ncols) {
+__device__ __forceinline__ int stage_cells(const ForceArgs<D>& A, const ForceParams& P,
+                                           const uint32_t* __restrict__ cs, TileSmem<D, V>& sm, int off, int ncell) {
     constexpr int R = TileRows<D>::R;
     constexpr int kT = TileCfg<D, V>::kTargets;
     constexpr int kPer = (TileCfg<D, V>::kCells + kT - 1) / kT;
     const int nx = P.g.nx;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int ncell = R * ncols;
     const int per = (ncell + kT - 1) / kT;
     int g0[kPer], len[kPer];
     int sum = 0;
@@ -241,7 +242,7 @@ __device__ __forceinline__ bool stage_columns(const ForceArgs<D>& A, const Force
         g0[i] = 0;
         len[i] = 0;
         if (i < per && e < ncell) {
-            const int ci = e / R, r = e - ci * R;
+            const int ci = (e + off) / R, r = e + off - ci * R;
             const int v = sm.colv[ci], row = sm.colrow[ci];
             int image = v < 0 ? kDownX : (v >= nx ? kUpX : 0);
             const int col = v < 0 ? v + nx : (v >= nx ? v - nx : v);
@@ -274,7 +275,22 @@ __device__ __forceinline__ bool stage_columns(const ForceArgs<D>& A, const Force
         before += w < warp ? x : 0;
         total += x;
     }
-    if (total > TileCfg<D, V>::kCap) return false;  // block-uniform
+    if (total > TileCfg<D, V>::kCap) {  // block-uniform
+        int fit = 0, end = before + inc - sum;
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+            const int e = tid * per + i;
+            end += len[i];
+            if (i < per && e < ncell && end <= TileCfg<D, V>::kCap) ++fit;
+        }
+        fit = __reduce_add_sync(kFull, fit);
+        if (lane == 0) sm.wcol[warp] = fit;
+        __syncthreads();
+        ncell = 0;
+#pragma unroll
+        for (int w = 0; w < kT / 32; ++w) ncell += sm.wcol[w];
+        if (ncell == 0) return 0;
+    }
     int run = before + inc - sum;
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
@@ -302,13 +318,13 @@ __device__ __forceinline__ bool stage_columns(const ForceArgs<D>& A, const Force
     }
     copy_wait();
     __syncthreads();
-    return true;
+    return ncell;
 }
 
 // Main force kernel (nx >= 3): one thread per target; a block takes
 // kTargets consecutive targets and stages their windows
-// so that each target reads one contiguous run (or, where a window does not
-// fit, reads the same cells from global memory).  Neighbouring threads mostly share a cell, hence a
+// so that each target reads one contiguous run (or one per part, or, where a
+// cell does not fit, the same cells from global memory).  Neighbouring threads mostly share a cell, hence a
 // window, so their candidate loads are broadcasts.  FP32 only: a target
 // whose neighbourhood holds a candidate that needs the FP64 decision is
 // deferred to its warp's closing pass (fixup_target), which recomputes it
@@ -452,32 +468,36 @@ __global__ void __launch_bounds__(TileCfg<D, V>::kTargets, TileCfg<D, V>::kMinBl
     const float* Mrow = M + (valid ? Layout<D>::type(me) : 0) * ms;
     Acc acc = {0.f, 0.f, 0.f, 0, 0ull, 0ull, 0ull};
     bool defer = false, direct = false;
-    // 2D, the whole warp together (a lane without `mine` takes no part).  The
-    // target's window: staged columns k .. k+2.  Only a target in the last
-    // column or row of a periodic box meets candidates flagged for a target
-    // shift; its whole warp then heeds the flags.
-    auto evaluate2 = [&](bool mine, int k, int ncell) {
+    // 2D, the whole warp together (a lane without `mine` takes no part): the
+    // target's staged cells lo .. up-1, its own cell being `own` (which may not
+    // be among them).  Only a target in the last column or row of a
+    // periodic box meets candidates flagged for a target shift; its whole warp
+    // then heeds the flags.
+    auto evaluate2 = [&](bool mine, int lo, int up, int own, int ncell) {
         const bool any_shift = __any_sync(kFull, mine && P.wrap && (cx == nx - 1 || cy == nx - 1));
         if (!mine) return;
-        const int j0 = sm.coff[k * R], j1 = sm.coff[(k + 3) * R];
-        const int own = (k + 1) * R + R / 2, o0 = sm.coff[own], o1 = sm.coff[own + 1];
-        const int self_j = o0 + (s - sm.cglob[own]);
-        defer = any_shift ? cand_window<D, DBG, true>(A, P, sm.cand, sm.coff, sm.cglob, Mrow, ncell, j0, o0, o1, j1,
-                                                      self_j, px, py, pz, acc)
-                          : cand_window<D, DBG, false>(A, P, sm.cand, sm.coff, sm.cglob, Mrow, ncell, j0, o0, o1, j1,
-                                                       self_j, px, py, pz, acc);
+        const int j0 = sm.coff[lo], j1 = sm.coff[up];
+        int o0 = j1, o1 = j1, self_j = -1;
+        if (lo <= own && own < up) {
+            o0 = sm.coff[own];
+            o1 = sm.coff[own + 1];
+            self_j = o0 + (s - sm.cglob[own]);
+        }
+        defer |= any_shift ? cand_window<D, DBG, true>(A, P, sm.cand, sm.coff, sm.cglob, Mrow, ncell, j0, o0, o1, j1,
+                                                       self_j, px, py, pz, acc)
+                           : cand_window<D, DBG, false>(A, P, sm.cand, sm.coff, sm.cglob, Mrow, ncell, j0, o0, o1, j1,
+                                                        self_j, px, py, pz, acc);
     };
     // 3D, the whole warp together (a lane without `mine` takes no part):
     // kCullWords words at a time, the distance test, then the kept
     // candidates' terms.
-    auto evaluate3 = [&](bool mine, int k, int ncell) {
+    auto evaluate3 = [&](bool mine, int lo, int up, int own, int ncell) {
         int j0 = 0, j1 = 0, self = -1;
         if (mine) {
-            j0 = sm.coff[k * R];
-            j1 = sm.coff[(k + 3) * R];
-            const int own = (k + 1) * R + R / 2;
-            self = sm.coff[own] + (s - sm.cglob[own]);
-            if (DBG) acc.cand += j1 - j0 - 1;
+            j0 = sm.coff[lo];
+            j1 = sm.coff[up];
+            if (lo <= own && own < up) self = sm.coff[own] + (s - sm.cglob[own]);
+            if (DBG) acc.cand += j1 - j0 - (self >= 0 ? 1 : 0);
         }
         // The lanes of a cell read the same candidates; the r-th cell of the
         // warp starts up to 7 before its window, at a staged index of r mod 8,
@@ -544,45 +564,45 @@ __global__ void __launch_bounds__(TileCfg<D, V>::kTargets, TileCfg<D, V>::kMinBl
             walk(std::true_type{});
         else
             walk(std::false_type{});
-        if (mine) defer = needs_fp64(K, umin);
+        if (mine) defer |= needs_fp64(K, umin);
     };
-    auto evaluate = [&](bool mine, int k, int ncell) {
+    auto evaluate = [&](bool mine, int lo, int up, int own, int ncell) {
         if constexpr (D == 3)
-            evaluate3(mine, k, ncell);
+            evaluate3(mine, lo, up, own, ncell);
         else
-            evaluate2(mine, k, ncell);
+            evaluate2(mine, lo, up, own, ncell);
     };
     const uint32_t* cs = A.cstart + P.cell_base;
-    // Stagings of the block's window columns [a, hi), each serving the
-    // targets whose window starts in [a, hi - 3]; one staging serves them all
-    // when every window fits.  A staging may span segments: its columns are
-    // staged one by one with their own rows, and a window never leaves its
-    // segment.  A staging whose candidates do not fit is retried with half as
-    // many columns (the width grows back after a success), and a single
-    // window that does not fit is read from global memory.  (Per-segment
-    // stagings served one segment per round: sparse 3D blocks spread over
-    // many grid rows.)
+    // Stagings of the block's stencil cells (R a column) one after another:
+    // [a, a + m) serves every target for the part of its window that lies in
+    // it, so a cell is staged once and all lanes of a crowded cell stay at
+    // work however few cells fit.  One staging serves them all when every
+    // window fits.  The parts follow in the window's order, hence the same
+    // bits.  A staging may span segments: its columns are staged one by one
+    // with their own rows, and a window never leaves its segment.  A cell that
+    // does not fit by itself sends the targets that need it to global memory.
+    // (Whole windows per staging, a window that did not fit read from global
+    // memory: 400k particles, 2D at 198 per cell, tile 1, 717 us a step, at
+    // 250 992; 3D at 50 per cell, tile 0, 825, tile 2 890.  In parts 589, 783,
+    // 560 and 587; whole columns per part 621, 820, 608 and 620.)
     constexpr int kCols = TileSmem<D, V>::kCols;
-    for (int a = 0, width = kCols; a <= ncol - 3;) {
-        const int hi = min(a + width, ncol);
-        fill_columns(a, hi);  // the previous staging no longer reads the columns
+    for (int a = 0; a < R * ncol;) {
+        const int c = a / R, off = a - c * R, hi = min(c + kCols, ncol);
+        fill_columns(c, hi);  // the previous staging no longer reads the columns
         __syncthreads();
-        const bool staged = stage_columns<D, V>(A, P, cs, sm, hi - a);
-        const bool mine = valid && kwin >= a && kwin <= hi - 3;
-        if (staged) {
-            evaluate(mine, kwin - a, R * (hi - a));
-            a = hi - 2;
-            width = min(kCols, 2 * width);
-        } else if (hi - a > 3) {
-            width = max(3, (hi - a) / 2);
-        } else {
-            if (mine) direct = true;  // computed after the loop, off the hot path
-            a += 1;
-        }
+        const int m = stage_cells<D, V>(A, P, cs, sm, off, R * (hi - c) - off);
+        const int lo = max(R * kwin - a, 0), up = min(R * (kwin + 3) - a, max(m, 1));
+        const bool mine = valid && !direct && lo < up;
+        if (m > 0)
+            evaluate(mine, lo, up, R * (kwin + 1) + R / 2 - a, m);
+        else
+            direct |= mine;  // computed after the loop, off the hot path
+        a += max(m, 1);
     }
     if (direct) {
-        // The window did not fit in shared memory: the same sum from global
-        // memory.
+        // A cell did not fit in shared memory: the same sum from global
+        // memory, in place of the parts summed so far.
+        acc = {0.f, 0.f, 0.f, 0, 0ull, 0ull, 0ull};
         defer = direct_stencil<D, DBG>(A, P, cs, Mrow, s, px, py, pz, cx, cy, cz, acc);
     }
     const bool done = valid && !defer;

@@ -1,0 +1,89 @@
+"""Windows staged in parts: crowded worlds whose windows exceed a staging, by
+cells that fit several at a time, one at a time, and not at all (those are
+read from global memory).  Every variant gives the bits of the others and the
+default one agrees with the oracle; and a candidate of a crowded window costs
+no more than a fixed multiple of what it costs where the windows fit."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from worlds import WorldSpec, compare_with_oracle, f32, rng_of, run_gpu_debug, uniform_world
+
+pytestmark = pytest.mark.gpu
+
+
+def _cluster(dim, n, wrap, seed):
+    """Two cells wide in every direction, around a corner of the box or (without wrapping) in the middle, with a
+    sparse rest, so that a block's columns are of all sizes."""
+    rng = rng_of(seed)
+    rmax = 0.05
+    pos = np.zeros((n, 3))
+    m = n - n // 8
+    p = rng.random((n, dim))
+    c = rng.uniform(-0.9 * rmax, 0.9 * rmax, (m, dim))
+    p[:m] = c - np.floor(c) if wrap else 0.5 + c
+    p = np.asarray(f32(p[rng.permutation(n)]), np.float32)
+    p[p >= 1.0] = 0.0
+    pos[:, :dim] = p
+    vel = np.zeros((n, 3))
+    vel[:, :dim] = f32(0.01 * rng.standard_normal((n, dim)))
+    types = rng.integers(0, 5, n).astype(np.int32)
+    return WorldSpec(dim, pos, vel, types, f32(rng.uniform(-1, 1, (5, 5))), rmax, dt=0.001, wrap=wrap)
+
+
+def _step(spec, variant, steps):
+    from plgpu.physics import GpuWorld
+
+    w = GpuWorld(spec.dim, spec.n)
+    try:
+        w.set_settings(spec.rmax, spec.friction, spec.force, spec.dt, beta=spec.beta, wrap=spec.wrap)
+        w.set_matrix(spec.matrix)
+        w.set_tile(variant)
+        w.upload(spec.pos, spec.vel, spec.types)
+        w.step(steps)
+        return w.download()
+    finally:
+        w.close()
+
+
+# A cell of the cluster holds a quarter or an eighth of it: windows of a few stagings, then cells on both sides of
+# each variant's staging.
+@pytest.mark.parametrize("wrap", [True, False])
+@pytest.mark.parametrize("dim,n", [(2, 1330), (2, 2640), (2, 5000), (2, 5500), (2, 6200), (2, 9700), (3, 1900), (3, 4100),
+                                   (3, 5100), (3, 7900), (3, 16700), (3, 20500)])
+def test_variants_agree(gpu, dim, n, wrap):
+    spec = _cluster(dim, n, wrap, 40 * dim + n)
+    states = [_step(spec, v, 2) for v in (0, 1, 2)]
+    for s in states[1:]:
+        for x, y in zip(s, states[0]):
+            assert np.array_equal(x, y)
+    if n <= 6200:  # beyond, the oracle's pairs take too long
+        compare_with_oracle(spec, *run_gpu_debug(spec))
+
+
+def _ns_per_candidate(dim, n, nx, variant):
+    from plgpu.physics import GpuWorld
+
+    spec = uniform_world(n, 6, 0.9999 / nx, seed=61, dim=dim)
+    w = GpuWorld(dim, n)
+    try:
+        w.set_settings(spec.rmax, spec.friction, spec.force, 1e-5, beta=spec.beta, wrap=spec.wrap)
+        w.set_matrix(spec.matrix)
+        w.set_tile(variant)
+        w.upload(spec.pos, spec.vel, spec.types)
+        w.step(2)
+        assert w.lib.plg_profile_enable(w.ctx, 1) == 0
+        w.step(6)
+        ms, launches = ctypes.c_double(), ctypes.c_int64()
+        assert w.lib.plg_profile_read(w.ctx, 3, ctypes.byref(ms), ctypes.byref(launches)) == 0
+        return 1e6 * ms.value / launches.value / (n * 3.0**dim * n / nx**dim)
+    finally:
+        w.close()
+
+
+# Particles per cell: windows that fit, and windows of more than the staging.  Best variant of each.
+@pytest.mark.parametrize("dim,n,fit,full", [(2, 400_000, 58, 40), (2, 400_000, 58, 34), (3, 400_000, 25, 20)])
+def test_crowded_windows_keep_the_rate(gpu, dim, n, fit, full):
+    best = [min(_ns_per_candidate(dim, n, nx, v) for v in (0, 1, 2)) for nx in (fit, full)]
+    assert best[1] <= 1.2 * best[0]
