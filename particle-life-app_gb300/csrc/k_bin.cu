@@ -476,7 +476,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(int n, int ncells,
                                                               uint32_t* zero_word) {
     extern __shared__ uint32_t small_smem[];
     uint32_t* const start = small_smem;              // first slot of each cell, ncells + 1
-    uint32_t* const next = start + ncells + 1;       // next free slot of each cell
+    uint32_t* const next = start + ncells + 1;       // next free slot of each of the block's cells
     uint32_t* const list = next + ncells;            // members of the block's cells, by slot - lo
     __shared__ uint32_t warp_sum[2][kSmallThreads / 32], crowd[kSmallCrowds], ncrowd;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -544,24 +544,23 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(int n, int ncells,
     uint32_t run = warp_sum[0][warp] + inc - sum;
     for (int c = c0; c < c1; ++c) {
         const uint32_t end = run + start[c];
-        if (end - run > kSmallCrowd && run < hi && end > lo) crowd[atomicAdd(&ncrowd, 1u)] = (uint32_t)c;
+        const bool crowded = end - run > kSmallCrowd;
+        if (crowded && run < hi && end > lo) crowd[atomicAdd(&ncrowd, 1u)] = (uint32_t)c;
         start[c] = run;
-        next[c] = run;
+        next[c] = !crowded && run >= lo && run < hi ? run : kNoMember;
         run = end;
     }
     if (tid == 0) start[ncells] = (uint32_t)n;
     __syncthreads();
-    auto move = [&](uint32_t i, uint32_t slot, uint32_t c) {
-        slot_cell[slot] = c;
-        b.pt[slot] = a.pt[i];
-        b.vel[slot] = a.vel[i];
+    auto put = [&](uint32_t slot, uint32_t c, float4 p, typename Layout<D>::Vel v) {
+        b.pt[slot] = p;
+        b.vel[slot] = v;
         if (cell_sorted) cell_sorted[slot] = (int32_t)c;
     };
     // The members of the block's cells, in any order within a cell.
     each4([&](int i, int m, uint4 q) {
         auto take = [&](int k, uint32_t c) {
-            if (k < m && start[c] >= lo && start[c] < hi && start[c + 1] - start[c] <= kSmallCrowd)
-                list[atomicAdd(next + c, 1u) - lo] = (uint32_t)(i + k);
+            if (k < m && next[c] != kNoMember) list[atomicAdd(next + c, 1u) - lo] = (uint32_t)(i + k);
         };
         take(0, q.x);
         take(1, q.y);
@@ -571,10 +570,14 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(int n, int ncells,
     __syncthreads();
     // Stable order within the cell: the members of a smaller index go first.
     if (tid < kSmallList && list[tid] != kNoMember) {
-        const uint32_t i = list[tid], c = cell[i], st = start[c], en = start[c + 1];
+        const uint32_t i = list[tid], c = cell[i];
+        const float4 p = a.pt[i];
+        const typename Layout<D>::Vel v = a.vel[i];
+        const uint32_t st = start[c], en = start[c + 1];
+        slot_cell[lo + tid] = c;
         uint32_t r = 0;
         for (uint32_t t = st - lo; t < en - lo; ++t) r += list[t] < i ? 1u : 0u;
-        move(i, st + r, c);
+        put(st + r, c, p, v);
     }
     // Crowded cells: their members in the order of the walk, those of this
     // block's slots moved.
@@ -596,7 +599,10 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(int n, int ncells,
 #pragma unroll
             for (int k = 0; k < 4; ++k)
                 if (is[k]) {
-                    if (slot >= lo && slot < hi) move((uint32_t)(i + k), slot, c);
+                    if (slot >= lo && slot < hi) {
+                        slot_cell[slot] = c;
+                        put(slot, c, a.pt[i + k], a.vel[i + k]);
+                    }
                     ++slot;
                 }
             first += __shfl_sync(kFull, w, 31);
