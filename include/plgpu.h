@@ -430,8 +430,10 @@ int plg_batch_step_stats(plg_batch* batch, int64_t* deferred);
  * 2D: 0 = 128 targets / 1152 staged candidates, 1 = 128 / 2048 (crowded
  * worlds), 2 = 128 / 1280 with more registers (small worlds); 3D: 0 = 128 /
  * 2176, 1 = 64 / 832 (sparse worlds), 2 = 128 / 1776 (large worlds).
- * All give the same bits.  Until a variant is set or tuned, a world joins
- * with variant 0, or 1 when it is a crowded 2D world (plg_set_tile).  Each world
+ * All give the same bits.  The worlds for which no variant was set or tuned
+ * are on variant 0, or on 1 while the whole batch consists of crowded 2D worlds
+ * (plg_set_tile).  After plg_batch_set_tile or plg_batch_autotune new worlds
+ * join with its variant.  Each world
  * of a batch has its own variant; a step launches the force kernel once per
  * variant in use.  The cell size is not a tuning choice: it is rmax (the
  * sorted order the reference exposes depends on it).  A single world has

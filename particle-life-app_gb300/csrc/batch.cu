@@ -45,6 +45,7 @@ struct WorldRec {
     int32_t steps_left = INT32_MAX;  // steps before the world freezes (INT32_MAX: no limit)
     bool dead = false;               // retired: frozen in place until the next compaction
     int variant = 0;                 // force kernel tile variant of this world
+    bool variant_set = false;        // set or tuned for this world (else assign_variants gives it)
 };
 
 }  // namespace
@@ -111,7 +112,7 @@ struct plg_batch {
     int64_t side_stage_cap = 0;
     int32_t next_id = 1;
     int variant = 0;  // tile variant given to new worlds (plg_batch_set_tile sets every world's)
-    bool variant_auto = true;  // neither set nor tuned: crowded worlds get the dense tile
+    bool variant_auto = true;  // not set or tuned for the whole batch (assign_variants)
     unsigned long long* wcycles_d = nullptr;  // wcap: per-world block cycles (per-world autotuner)
     void* tune_save[5] = {};                  // the tuners' copy of the state (kept, grown on demand)
     size_t tune_cap[5] = {};
@@ -281,9 +282,21 @@ int check_desc(plg_batch* b, const plg_world_desc& d) {
     return rc ? berr(b, rc, msg) : PLG_OK;
 }
 
-// The tile variant of a world that joins.
-int new_world_variant(const plg_batch* b, const WorldRec& w) {
-    return b->variant_auto && crowded_world(b->dim, w.n, w.ncells) ? 1 : b->variant;
+// The tile variant of the worlds for which none was set or tuned, whenever
+// the membership changes: the dense one where the whole batch is crowded, so
+// that it never opens a second force launch.  That costs every step more than
+// the dense tile gives the crowded worlds of a mixed batch, but for the largest
+// (a fork and join, and no chaining of steps).  15 worlds of 3,000 to 10,000
+// particles and one of n at d per cell, dense tile for that one against one
+// launch: n 432, d 48: 34.7 / 33.5 us a step; 5,000, 62: 51.4 / 47.2; 50,000,
+// 80: 80.7 / 78.6; 200,000, 125: 232 / 246; 20,000 in blobs, 62: 332 / 307.
+void assign_variants(plg_batch* b) {
+    if (!b->variant_auto) return;
+    bool crowded = true;
+    for (const WorldRec& w : b->worlds)
+        if (!w.dead && w.n > 0) crowded &= w.variant_set ? w.variant == 1 : crowded_world(b->dim, w.n, w.ncells);
+    for (WorldRec& w : b->worlds)
+        if (!w.variant_set) w.variant = crowded ? 1 : b->variant;
 }
 
 // The force kernel's tile tables: for each variant v, the first tile of
@@ -369,6 +382,7 @@ int upload_tables(plg_batch* b) {
     if (nw) BCK(b, cudaMemcpyAsync(b->steps_left_d, left.data(), sizeof(int) * nw, cudaMemcpyHostToDevice, b->stream));
     // The host vectors die at return: wait for the copies.
     BCK(b, cudaStreamSynchronize(b->stream));
+    assign_variants(b);
     return write_tiles(b);
 }
 
@@ -405,7 +419,7 @@ int relayout(plg_batch* b, const std::vector<int>& survivors, const plg_world_de
         w.s = d.settings;
         w.nx = grid_n(d.settings.rmax);
         w.ncells = (int64_t)w.nx * w.nx * (D == 3 ? w.nx : 1);
-        w.variant = new_world_variant(b, w);
+        w.variant = b->variant;
         w.bounds.resize((size_t)w.nx + 1);
         build_bounds(d.settings.rmax, w.nx, w.bounds.data());
         w.matrix.resize((size_t)d.ntypes * d.ntypes);
@@ -649,7 +663,7 @@ int append_world(plg_batch* b, const plg_world_desc& d, const WorldGen* gen, int
     w.s = d.settings;
     w.nx = grid_n(d.settings.rmax);
     w.ncells = (int64_t)w.nx * w.nx * (D == 3 ? w.nx : 1);
-    w.variant = new_world_variant(b, w);
+    w.variant = b->variant;
     const int64_t nbounds = w.nx + 1, nmat = (int64_t)d.ntypes * d.ntypes;
     if (b->n_total + b->pend_n + w.n > b->pcap) return berr(b, PLG_E_CAPACITY, "batch particle capacity exceeded");
     if (b->c_total + b->pend_c + w.ncells > b->ccap) return berr(b, PLG_E_CAPACITY, "batch cell capacity exceeded");
@@ -1114,6 +1128,7 @@ int plg_batch_set_world_tile(plg_batch* b, int32_t id, int32_t variant) {
     if (variant < 0 || variant >= PLG_TILE_VARIANTS) return berr(b, PLG_E_INVALID_ARG, "unknown tile variant");
     const int k = find_world(b, id);
     if (k < 0) return berr(b, PLG_E_INVALID_ARG, "unknown world id " + std::to_string(id));
+    b->worlds[(size_t)k].variant_set = true;
     if (b->worlds[(size_t)k].variant == variant) return PLG_OK;
     BatchDeviceGuard g(b->device);
     b->worlds[(size_t)k].variant = variant;
@@ -1226,8 +1241,8 @@ void set_all_variants(plg_batch* b, int v) {
 
 // Times `steps` steps of each tile variant on the batch as it is, restoring
 // the particle state after each trial, and gives every world the fastest
-// variant.  The trials allocate a copy of the state and free it before
-// returning.
+// variant.  The trials work on a copy of the state that the batch keeps for
+// the next tuning.
 int plg_batch_autotune(plg_batch* b, int32_t steps, int32_t* chosen, double* ms_per_step) {
     if (!b) return PLG_E_INVALID_ARG;
     if (steps < 1) return berr(b, PLG_E_INVALID_ARG, "autotune needs at least one step");
@@ -1242,7 +1257,10 @@ int plg_batch_autotune(plg_batch* b, int32_t steps, int32_t* chosen, double* ms_
     TrialState ts(b);
     int rc = ts.alloc();
     if (!rc) rc = ts.copy(false);
-    const int old = b->variant;
+    // The variant to beat: the one the worlds are on, where they share one.
+    int old = before[0];
+    for (int v : before)
+        if (v != old) old = b->variant;
     double times[PLG_TILE_VARIANTS] = {};
     int best_v = old;
     double best = 1e300;
@@ -1338,6 +1356,7 @@ int plg_batch_autotune_worlds(plg_batch* b, int32_t steps, int32_t* variants, do
         for (int v = 0; v < PLG_TILE_VARIANTS; ++v) ms_by_variant[v] = uni[v];
         ms_by_variant[PLG_TILE_VARIANTS] = mixed;
     }
+    for (WorldRec& w : b->worlds) w.variant_set = true;
     if (variants)
         for (size_t k = 0; k < nw; ++k) variants[k] = b->worlds[k].variant;
     return PLG_OK;

@@ -407,9 +407,10 @@ inline int switch_if_faster(int current, int best, const double* ms_per_step) {
 int tile_targets(int dim, int variant);
 
 // A 2D world with this many particles per cell on average takes the dense
-// tile (variant 1) until a variant is set or tuned: it is 2% ahead at 60 per
-// cell and 34% at 119, and a clustered world is only denser where its
-// particles are.
+// tile (variant 1) until a variant is set or tuned: 400k particles, a step,
+// variant 0 against 1: 119 per cell 375 / 337 us, 198 per cell 635 / 589, 250
+// 810 / 783, 309 equal; a clustered world is only denser where its particles
+// are.  (In a batch: assign_variants.)
 constexpr int64_t kCrowdedCell2D = 48;
 inline bool crowded_world(int dim, int64_t n, int64_t ncells) { return dim == 2 && n >= kCrowdedCell2D * ncells; }
 
