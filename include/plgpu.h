@@ -429,7 +429,7 @@ int plg_batch_step_stats(plg_batch* batch, int64_t* deferred);
 /* Force kernel tile variants (threads = targets per block, staging size):
  * 2D: 0 = 128 targets / 1152 staged candidates, 1 = 128 / 2048 (crowded
  * worlds), 2 = 128 / 1280 with more registers (small worlds); 3D: 0 = 128 /
- * 2176, 1 = 64 / 832 (sparse worlds), 2 = 128 / 1776 (large worlds).
+ * 2176, 1 = 64 / 944 (sparse worlds), 2 = 128 / 1776 (large worlds).
  * All give the same bits.  The worlds for which no variant was set or tuned
  * are on variant 0, or on 1 while the whole batch consists of crowded 2D worlds
  * (plg_set_tile).  After plg_batch_set_tile or plg_batch_autotune new worlds

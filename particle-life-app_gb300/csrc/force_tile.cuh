@@ -149,7 +149,10 @@ __global__ void __launch_bounds__(kThreads) k_force_general(const __grid_constan
 // 3D: 71 staged columns of 9 cells in variants 0 and 2, so that the sparse
 // tails of a blob world stage in one or two rounds.  Variant 0: 4 blocks of
 // 128 targets with 2176 candidates, for dense cells and for worlds of about
-// one wave.  Variant 1: the smaller tile for small sparse worlds.  Variant 2:
+// one wave.  Variant 1: the smaller tile for small sparse worlds, 9 blocks of
+// 64 targets with the candidates their shared memory holds (asking for 10,
+// which did not fit beside 832 candidates, 9 ran with too few registers: 250k
+// uniform 95 us, now 90; 10 blocks of 808 candidates 96).  Variant 2:
 // 5 blocks of 128 targets with 1776 candidates, as much shared memory as five
 // blocks have, for large worlds (4M in blobs 1066 us against variant 0's 1148;
 // with 448 cells it took 1108, with 832 cells and 1600 candidates 1124; 1M at
@@ -175,7 +178,7 @@ struct TileCfg<3, 0> {
 };
 template <>
 struct TileCfg<3, 1> {
-    static constexpr int kTargets = 64, kMinBlocks = 10, kCap = 832, kCells = 320;
+    static constexpr int kTargets = 64, kMinBlocks = 9, kCap = 944, kCells = 320;
 };
 template <>
 struct TileCfg<3, 2> {
@@ -207,6 +210,15 @@ struct TileSmem {
     float mat[kSmemMatrixMax * smem_matrix_stride<D>(kSmemMatrixMax)];
     uint8_t image[TileCfg<D, V>::kCells];  // image shifts of stencil cell e (kUp*, kDown*)
 };
+
+// The blocks per SM that a variant asks for fit into an SM's shared memory:
+// 228 KB, in units of 128 bytes, and 1 KB more per block.
+template <int D, int V>
+constexpr bool blocks_fit() {
+    return TileCfg<D, V>::kMinBlocks * ((sizeof(TileSmem<D, V>) + 127) / 128 * 128 + 1024) <= 228 * 1024;
+}
+static_assert(blocks_fit<2, 0>() && blocks_fit<2, 1>() && blocks_fit<2, 2>(), "2D tile");
+static_assert(blocks_fit<3, 0>() && blocks_fit<3, 1>() && blocks_fit<3, 2>(), "3D tile");
 
 // Stages ncell cells of the listed columns (sm.colv, sm.colrow), from cell
 // `off` of the first one on, column-major: for each column the cells of its R

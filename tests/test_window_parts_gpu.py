@@ -51,7 +51,7 @@ def _step(spec, variant, steps):
 # each variant's staging.
 @pytest.mark.parametrize("wrap", [True, False])
 @pytest.mark.parametrize("dim,n", [(2, 1330), (2, 2640), (2, 5000), (2, 5500), (2, 6200), (2, 9700), (3, 1900), (3, 4100),
-                                   (3, 5100), (3, 7900), (3, 16700), (3, 20500)])
+                                   (3, 5100), (3, 7900), (3, 8900), (3, 16700), (3, 20500)])
 def test_variants_agree(gpu, dim, n, wrap):
     spec = _cluster(dim, n, wrap, 40 * dim + n)
     states = [_step(spec, v, 2) for v in (0, 1, 2)]
