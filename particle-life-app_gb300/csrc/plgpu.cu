@@ -346,23 +346,23 @@ void enqueue_body(plg_ctx* c, const DebugOut* dbg, int32_t* cell_sorted, const H
     uint32_t* const zero_word = c->general ? nullptr : c->defer;
     const bool small = sort_is_small(n, c->ncells);
     k0(PLG_K_SCAN);
-    if (small)  // the whole sort (profiled as the scan)
+    if (small)  // the whole sort, profiled as the scan: it has no scatter and no gather
         launch_sort_small<D>(st, n, c->ncells, c->cell, c->counts, c->cstart, c->slot_cell, buf_a<D>(c), buf_b<D>(c),
                              cell_sorted, zero_word, !c->profiling);
     else
         launch_scan(st, c->counts, c->ncells, c->cstart, c->scan_state, c->status_d, zero_word, !c->profiling);
     k1(PLG_K_SCAN);
-    k0(PLG_K_SCATTER);
     if (!small) {
+        k0(PLG_K_SCATTER);
         if (n > 0)
             launch_scatter(st, n, c->cell, c->counts, c->cstart, c->perm, c->slot_cell, c->scan_state, nstate);
         else
             cudaMemsetAsync(c->scan_state, 0, sizeof(unsigned long long) * (size_t)nstate, st);
+        k1(PLG_K_SCATTER);
+        k0(PLG_K_GATHER);
+        launch_gather<D>(st, n, c->perm, c->slot_cell, c->cstart, buf_a<D>(c), buf_b<D>(c), cell_sorted);
+        k1(PLG_K_GATHER);
     }
-    k1(PLG_K_SCATTER);
-    k0(PLG_K_GATHER);
-    if (!small) launch_gather<D>(st, n, c->perm, c->slot_cell, c->cstart, buf_a<D>(c), buf_b<D>(c), cell_sorted);
-    k1(PLG_K_GATHER);
     k0(PLG_K_FORCE);
     launch_force<D>(st, c->fp, c->general, buf_b<D>(c), c->cstart, c->slot_cell, buf_a<D>(c), c->cell, c->counts,
                     c->defer, dbg, tile_variant(c), snap);
@@ -398,7 +398,9 @@ int enqueue_rebin(plg_ctx* c) {
 
 int accumulate_profile(plg_ctx* c) {
     CK(c, cudaEventSynchronize(c->pev[PLG_K_COUNT - 1][1]));  // the step's last kernel
+    const bool small = sort_is_small((int)c->n, c->ncells);
     for (int k = 0; k < PLG_K_COUNT; ++k) {
+        if (small && (k == PLG_K_SCATTER || k == PLG_K_GATHER)) continue;  // no such launch (enqueue_body)
         float ms = 0.f;
         CK(c, cudaEventElapsedTime(&ms, c->pev[k][0], c->pev[k][1]));
         c->prof_ms[k] += ms;
