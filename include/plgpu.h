@@ -121,9 +121,11 @@ int plg_upload(plg_ctx* ctx, int64_t n, const double* pos, const double* vel,
                const int32_t* type);
 
 /* nsteps x Physics.update() (Physics.java:112-134).  Blocks until done.
- * Checks the stop flag between steps (every fourth step in long calls on
- * worlds of up to 524,288 particles): a set flag ends the call early with
- * PLG_E_STOPPED and is cleared (Physics.forceUpdateStop, Physics.java:149). */
+ * Checks the stop flag before each step that it enqueues, on worlds of up to
+ * 524,288 particles before each four: a set flag ends the call early with
+ * PLG_E_STOPPED and is cleared (Physics.forceUpdateStop, Physics.java:149).
+ * The steps enqueued by then are still done: at most eight on worlds of up to
+ * 524,288 particles, at most four on larger ones. */
 int plg_step(plg_ctx* ctx, int32_t nsteps);
 
 /* Enqueues nsteps without waiting; pair with plg_sync. */
@@ -278,7 +280,8 @@ int plg_permute(plg_ctx* ctx, int64_t n_new, const int32_t* src);
 int plg_set_types(plg_ctx* ctx, const int32_t* type);
 
 /* Thread-safe stop request: Physics.forceUpdateStop (Physics.java:149-151)
- * and Physics.kill (Physics.java:156-158).  Takes effect between steps. */
+ * and Physics.kill (Physics.java:156-158).  Takes effect between steps, with
+ * the steps already enqueued still done (plg_step). */
 int plg_request_stop(plg_ctx* ctx);
 
 /* Message of the last failing call on this context ("" if none). */
@@ -288,7 +291,8 @@ const char* plg_last_error(plg_ctx* ctx);
  * can order its own work and record CUDA events against it. */
 int plg_get_stream(plg_ctx* ctx, void** stream);
 
-/* 1 (default): each step is one CUDA graph launch.  0: plain launches. */
+/* 1 (default): steps are CUDA graph launches, of one step or of four (long
+ * calls, plg_step).  0: plain launches. */
 int plg_set_use_graph(plg_ctx* ctx, int32_t on);
 
 /* ---- measurement ------------------------------------------------------ */

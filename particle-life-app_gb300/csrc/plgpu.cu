@@ -86,13 +86,15 @@ void fill_force_params(const plg_settings& s, int nx, int64_t ncells, int ntypes
 
 namespace {
 
-constexpr int kRing = 4;  // steps (or graphs of kGraphSteps steps) in flight per plg_step call
+constexpr int kRing = 4;  // launches (of one step or of kGraphSteps) in flight per plg_step call
 // A graph of several steps keeps the programmatic edge from one step's force
 // kernel to the next step's sort and saves the gap between graphs: 3.5 to 4 us
 // a step (10k particles 18.2 -> 14.6 us, 120k 49 -> 45, 1M 92.8 -> 91.2).  It is
 // the unit in which a stop request is answered, so larger worlds, which gain
-// little, step one by one.
-constexpr int kGraphSteps = 4;
+// little, step one by one, and no more than two graphs' steps are in flight
+// (four graphs gain nothing: the device is busy with one while the host
+// launches the other).
+constexpr int kGraphSteps = 4, kFlightSteps = 2 * kGraphSteps;
 constexpr int64_t kManyParticles = 1 << 19;
 constexpr size_t kRenderKeep = (size_t)64 << 20;  // render buffers kept between calls
 
@@ -224,7 +226,8 @@ struct plg_ctx {
     double prof_ms[PLG_K_COUNT] = {};
     int64_t prof_n[PLG_K_COUNT] = {};
 
-    cudaEvent_t ring[kRing] = {};
+    cudaEvent_t ring[kRing] = {};  // the launches in flight, each with its steps
+    int ring_steps[kRing] = {};
     int ring_pos = 0;
     int ring_fill = 0;
 
@@ -762,19 +765,20 @@ int plg_step_async(plg_ctx* c, int32_t nsteps) {
     if (nsteps < 0) return set_err(c, PLG_E_INVALID_ARG, "negative step count");
     DeviceGuard g(c->device);
     for (int32_t k = 0; k < nsteps;) {
-        if (c->stop.exchange(0)) return set_err(c, PLG_E_STOPPED, "stopped by plg_request_stop");
-        if (c->ring_fill == kRing) {
-            CK(c, cudaEventSynchronize(c->ring[c->ring_pos]));
+        const int m = many_steps(c, nsteps - k) ? kGraphSteps : 1;
+        // Room for m steps: the oldest launches end first.
+        for (;;) {
+            int flight = 0;
+            for (int i = 1; i <= c->ring_fill; ++i) flight += c->ring_steps[(c->ring_pos + kRing - i) % kRing];
+            if (c->ring_fill < kRing && flight + m <= kFlightSteps) break;
+            CK(c, cudaEventSynchronize(c->ring[(c->ring_pos + kRing - c->ring_fill) % kRing]));
             c->ring_fill--;
         }
-        if (many_steps(c, nsteps - k)) {
-            if ((rc = launch_step_graph(c, kGraphSteps))) return rc;
-            k += kGraphSteps;
-        } else {
-            if ((rc = enqueue_step(c))) return rc;
-            ++k;
-        }
+        if (c->stop.exchange(0)) return set_err(c, PLG_E_STOPPED, "stopped by plg_request_stop");
+        if ((rc = m > 1 ? launch_step_graph(c, m) : enqueue_step(c))) return rc;
+        k += m;
         CK(c, cudaEventRecord(c->ring[c->ring_pos], c->stream));
+        c->ring_steps[c->ring_pos] = m;
         c->ring_pos = (c->ring_pos + 1) % kRing;
         c->ring_fill++;
     }
