@@ -196,9 +196,12 @@ constexpr int kCullWords = 8;
 template <int D, int V>
 struct TileSmem {
     static constexpr int kCols = TileCfg<D, V>::kCells / TileRows<D>::R;
-    float4 before[D == 3 ? 8 : 1];         // read by the 3D distance test, never kept
-    float4 cand[TileCfg<D, V>::kCap + (D == 3 ? kCullGroup : 0)];  // staged candidates, column-major by stencil cell
-    int coff[TileCfg<D, V>::kCells + 1];   // smem start of stencil cell e = column * R + row
+    // Staged candidates, column-major by stencil cell, from index kLead on.
+    // The 3D distance test also reads the kLead entries before them and up to
+    // a group after them, and keeps none of those.
+    static constexpr int kLead = D == 3 ? 8 : 0;
+    float4 slots[kLead + TileCfg<D, V>::kCap + (D == 3 ? kCullGroup : 0)];
+    int coff[TileCfg<D, V>::kCells + 1];   // staged start of stencil cell e = column * R + row
     int cglob[TileCfg<D, V>::kCells];      // sorted-order start of stencil cell e
     int colv[kCols];                       // virtual column of staged column ci
     int colrow[kCols];                     // grid row of staged column ci: y, or y | z << 16
@@ -320,7 +323,7 @@ __device__ __forceinline__ int stage_cells(const ForceArgs<D>& A, const ForcePar
     for (int e = tid >> lg; e < ncell; e += kT >> lg) {
         const int d = sm.coff[e], m = sm.coff[e + 1] - d, image = sm.image[e];
         const float4* __restrict__ src = A.bpt + sm.cglob[e];
-        float4* dst = sm.cand + d;
+        float4* dst = sm.slots + TileSmem<D, V>::kLead + d;
         int k = tid & ((1 << lg) - 1);
         if (image) {
             for (; k < m; k += 1 << lg) dst[k] = shift_candidate<D>(__ldg(src + k), image);
@@ -477,6 +480,7 @@ __global__ void __launch_bounds__(TileCfg<D, V>::kTargets, TileCfg<D, V>::kMinBl
     };
     const int nx = P.g.nx;
     const float px = me.x, py = me.y, pz = D == 3 ? me.z : 0.f;
+    const float4* const cand = sm.slots + TileSmem<D, V>::kLead;
     const float* Mrow = M + (valid ? Layout<D>::type(me) : 0) * ms;
     Acc acc = {0.f, 0.f, 0.f, 0, 0ull, 0ull, 0ull};
     bool defer = false, direct = false;
@@ -495,9 +499,9 @@ __global__ void __launch_bounds__(TileCfg<D, V>::kTargets, TileCfg<D, V>::kMinBl
             o1 = sm.coff[own + 1];
             self_j = o0 + (s - sm.cglob[own]);
         }
-        defer |= any_shift ? cand_window<D, DBG, true>(A, P, sm.cand, sm.coff, sm.cglob, Mrow, ncell, j0, o0, o1, j1,
+        defer |= any_shift ? cand_window<D, DBG, true>(A, P, cand, sm.coff, sm.cglob, Mrow, ncell, j0, o0, o1, j1,
                                                        self_j, px, py, pz, acc)
-                           : cand_window<D, DBG, false>(A, P, sm.cand, sm.coff, sm.cglob, Mrow, ncell, j0, o0, o1, j1,
+                           : cand_window<D, DBG, false>(A, P, cand, sm.coff, sm.cglob, Mrow, ncell, j0, o0, o1, j1,
                                                         self_j, px, py, pz, acc);
     };
     // 3D, the whole warp together (a lane without `mine` takes no part):
@@ -531,7 +535,7 @@ __global__ void __launch_bounds__(TileCfg<D, V>::kTargets, TileCfg<D, V>::kMinBl
                 int n = 0;
                 for (int i = 0; i < nw; ++i) {
                     const int base = j + 32 * i;
-                    uint32_t m = cull_word<kShifted>(sm.cand + base, min(32, j1 - base), px, py, pz, neg_thr);
+                    uint32_t m = cull_word<kShifted>(cand + base, min(32, j1 - base), px, py, pz, neg_thr);
                     if (base < j0) m &= kFull >> (j0 - base);
                     if ((unsigned)(self - base) < 32u) m &= ~(0x80000000u >> (self - base));
                     if (m) {
@@ -552,7 +556,7 @@ __global__ void __launch_bounds__(TileCfg<D, V>::kTargets, TileCfg<D, V>::kMinBl
                     }
                     const int b = top_bit(m);
                     m &= (1u << b) - 1u;
-                    const float4 q = sm.cand[top - b];
+                    const float4 q = cand[(int)top - b];
                     int tb = __float_as_int(q.w);
                     float pxe = px, pye = py, pze = pz;
                     if (kShifted) {
