@@ -494,7 +494,7 @@ __global__ void __launch_bounds__(TileCfg<D, V>::kTargets, TileCfg<D, V>::kMinBl
         if (!mine) return;
         const int j0 = sm.coff[lo], j1 = sm.coff[up];
         int o0 = j1, o1 = j1, self_j = -1;
-        if (lo <= own && own < up) {
+        if ((unsigned)(own - lo) < (unsigned)(up - lo)) {
             o0 = sm.coff[own];
             o1 = sm.coff[own + 1];
             self_j = o0 + (s - sm.cglob[own]);
@@ -512,7 +512,7 @@ __global__ void __launch_bounds__(TileCfg<D, V>::kTargets, TileCfg<D, V>::kMinBl
         if (mine) {
             j0 = sm.coff[lo];
             j1 = sm.coff[up];
-            if (lo <= own && own < up) self = sm.coff[own] + (s - sm.cglob[own]);
+            if ((unsigned)(own - lo) < (unsigned)(up - lo)) self = sm.coff[own] + (s - sm.cglob[own]);
             if (DBG) acc.cand += j1 - j0 - (self >= 0 ? 1 : 0);
         }
         // The lanes of a cell read the same candidates; the r-th cell of the
@@ -607,13 +607,16 @@ __global__ void __launch_bounds__(TileCfg<D, V>::kTargets, TileCfg<D, V>::kMinBl
         fill_columns(c, hi);  // the previous staging no longer reads the columns
         __syncthreads();
         const int m = stage_cells<D, V>(A, P, cs, sm, off, R * (hi - c) - off);
-        const int lo = max(R * kwin - a, 0), up = min(R * (kwin + 3) - a, max(m, 1));
-        const bool mine = valid && !direct && lo < up;
-        if (m > 0)
-            evaluate(mine, lo, up, R * (kwin + 1) + R / 2 - a, m);
-        else
-            direct |= mine;  // computed after the loop, off the hot path
-        a += max(m, 1);
+        const int w = R * kwin - a;  // the window's first cell in this staging
+        const int lo = max(w, 0);
+        if (m > 0) {
+            const int up = min(w + 3 * R, m);
+            evaluate(valid && lo < up, lo, up, w + R + R / 2, m);
+            a += m;
+        } else {
+            direct |= valid && w <= 0 && w + 3 * R > 0;  // computed after the loop, off the hot path
+            ++a;
+        }
     }
     if (direct) {
         // A cell did not fit in shared memory: the same sum from global
