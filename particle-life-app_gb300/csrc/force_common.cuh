@@ -1,9 +1,9 @@
 // force_common.cuh — the building blocks of the force kernels (force_tile.cuh):
 // kernel arguments, the FP64 pair decision and term, the candidate
-// evaluation over a staged window, the global-memory stencils (the direct
-// path and the deferred FP64 pass) and the epilogue.  Every path evaluates a
-// target's candidates in the same order with the same arithmetic, so they
-// give the same bits.
+// evaluation over a staged window, the global-memory stencil of the deferred
+// FP64 pass and the epilogue.  Every tile shape evaluates a target's
+// candidates in the same order with the same arithmetic, so they give the
+// same bits.
 #pragma once
 
 #include <climits>
@@ -459,8 +459,7 @@ struct LoopK {
 
 // One candidate: d = q - p with the image shifts already applied to q and p,
 // the FP32 Accelerator term added to acc, and umin = min(umin, |u|) (NaN
-// sticks).  The staged and the direct paths both use it, in the same
-// candidate order, so they produce the same bits.  Returns d2.
+// sticks).  Returns d2.
 //
 // Force law in FP32, with inv = 1/|d| (rsqrt.approx) and u+ = max(u, 0):
 //   below beta rmax   f/|d| = 1/(beta rmax) - 1/|d|   (u+ = 0 there)
@@ -606,7 +605,7 @@ __device__ __forceinline__ bool cand_window(const ForceArgs<D>& A, const ForcePa
 // exact zero and has |u| far from zero, so sums and deferrals have the same
 // bits as a walk over all candidates.  (One loop forming every term: about
 // 20 instructions a candidate, issue and shared-memory pipe both at 62-70%.
-// Now 10 a candidate for the test, bound by the shared-memory pipe, and 42 a
+// Now 7.5 a candidate for the test, bound by the shared-memory pipe, and 42 a
 // kept candidate: force kernel of 250k uniform particles 118 -> 87 us, of 4M
 // in blobs 1187 -> 1169 us, of 1M with 50 neighbours 416 -> 323 us.)
 constexpr float kCullRel = 1.6e-5f;
@@ -649,94 +648,6 @@ __device__ __forceinline__ uint32_t cull_word(const float4* __restrict__ cand, i
     }
     m <<= 32 - c;
     return n < 32 ? m & ~(kFull >> n) : m;
-}
-
-// The target's neighbourhood read straight from global memory, for windows
-// with a cell too full for shared memory: the cells in the staged order
-// (columns cx-1..cx+1, and in each the R stencil rows), the same image
-// shifts (below the box: the candidate's coordinate minus 1; above: the
-// target's) and the same candidate evaluation, so the sum has the same bits
-// as the staged path would give.
-// Eight candidates per trip, their loads and terms independent, added in
-// candidate order: one at a time, a trip waited for its own load (clustered
-// worlds, a step: 100k 2D particles in blobs of 0.006 665 -> 333 us, 500k 3D
-// in blobs of 0.04 2214 -> 1373; four per trip 391 and 1495).
-template <int D, bool DBG>
-__device__ __noinline__ bool direct_stencil(const ForceArgs<D>& A, const ForceParams& P,
-                                            const uint32_t* __restrict__ cs, const float* __restrict__ Mrow, int s,
-                                            float px, float py, float pz, int cx, int cy, int cz, Acc& acc) {
-    constexpr int R = D == 3 ? 9 : 3;
-    const LoopK K(P);
-    const int nx = P.g.nx;
-    const bool wrap = P.wrap != 0;
-    float umin = INFINITY;
-    for (int ci = 0; ci < 3; ++ci) {
-        int col = cx - 1 + ci;
-        bool qsx = false, tsx = false;
-        if (col < 0) {
-            col += nx;
-            qsx = wrap;
-        } else if (col >= nx) {
-            col -= nx;
-            tsx = wrap;
-        }
-        const float pxe = tsx ? px - 1.f : px;
-        for (int r = 0; r < R; ++r) {
-            int ry = cy + r % 3 - 1, rz = D == 3 ? cz + r / 3 - 1 : 0;
-            bool qsy = false, qsz = false;
-            float pye = py, pze = pz;
-            if (ry < 0) {
-                ry += nx;
-                qsy = wrap;
-            } else if (ry >= nx) {
-                ry -= nx;
-                if (wrap) pye = py - 1.f;
-            }
-            if (D == 3) {
-                if (rz < 0) {
-                    rz += nx;
-                    qsz = wrap;
-                } else if (rz >= nx) {
-                    rz -= nx;
-                    if (wrap) pze = pz - 1.f;
-                }
-            }
-            const int c = (rz * nx + ry) * nx + col;
-            const int j0 = (int)__ldg(cs + c), j1 = (int)__ldg(cs + c + 1);
-            const int self = ci == 1 && r == R / 2 ? s : -1;
-            const float sx = qsx ? 1.f : 0.f, sy = qsy ? 1.f : 0.f, sz = qsz ? 1.f : 0.f;
-            auto term = [&](int j) {
-                float4 q = __ldg(A.bpt + j);
-                if (j == self) q.x += 8.f;  // an exact zero term (cand_window)
-                const int t = Layout<D>::type(q);
-                return cand_term<D>(K, q.x - sx, q.y - sy, D == 3 ? q.z - sz : 0.f, pxe, pye, pze, Mrow[t], umin);
-            };
-            auto count = [&](int j, float d2) {
-                if (DBG && j != self) {
-                    acc.cand++;
-                    if ((d2 <= K.lo) & (d2 > 0.f))
-                        add_pair<D, true>(acc, make_float4(0.f, 0.f, 0.f, 0.f), id_of<D>(A, j));
-                }
-            };
-            constexpr int U = 8;
-            int j = j0;
-            for (; j + U <= j1; j += U) {
-                Term<D> t[U];
-#pragma unroll
-                for (int k = 0; k < U; ++k) t[k] = term(j + k);
-#pragma unroll
-                for (int k = 0; k < U; ++k) add_term<D>(acc, t[k]);
-#pragma unroll
-                for (int k = 0; k < U; ++k) count(j + k, t[k].d2);
-            }
-            for (; j < j1; ++j) {
-                const Term<D> t = term(j);
-                add_term<D>(acc, t);
-                count(j, t.d2);
-            }
-        }
-    }
-    return needs_fp64(K, umin);
 }
 
 // Sum of `v` over the warp in a fixed butterfly order (the same bits on

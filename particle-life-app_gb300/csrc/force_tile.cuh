@@ -19,11 +19,10 @@
 // memory column by column, each column's R cells in turn, so that every
 // target's neighbourhood is one contiguous run.  When the whole block's
 // windows fit, one staging serves every target; otherwise the block's
-// cells are staged in parts, as many at a time as fit, and each part serves
-// every target whose window meets it.  A cell that does not fit by itself
-// (a very dense region) sends the targets that need it to global memory
-// (direct_stencil).  The candidates come in the same order and give the same
-// bits throughout.  The 2D
+// cells are staged in parts, as many at a time as fit (of a cell that does not
+// fit by itself, a slice), and each part serves every target whose window
+// meets it.  The candidates come in the same order and give the same bits
+// throughout.  The 2D
 // candidate loop is branch-free FP32; a 3D window is tested by distance
 // first, and terms are formed for what that keeps.  A target that meets a
 // candidate needing the FP64 decision is deferred: its warp recomputes it from global
@@ -226,7 +225,8 @@ static_assert(blocks_fit<3, 0>() && blocks_fit<3, 1>() && blocks_fit<3, 2>(), "3
 // Stages ncell cells of the listed columns (sm.colv, sm.colrow), from cell
 // `off` of the first one on, column-major: for each column the cells of its R
 // stencil rows in turn, so that the neighbourhood of a target whose window
-// starts at column k is the single contiguous range of columns k .. k+2.  Images below the box are
+// starts at column k is the single contiguous range of columns k .. k+2;
+// without the first `skip` members of the first cell.  Images below the box are
 // shifted down by 1 here (exact: their coordinates are >= 0.5); images above
 // it are flagged for a target shift instead.  Thread t places cells
 // t*per .. t*per+per-1: it reads their extents, and the block scans the
@@ -237,12 +237,14 @@ static_assert(blocks_fit<3, 0>() && blocks_fit<3, 1>() && blocks_fit<3, 2>(), "3
 // staging and the target rows without integer divisions, together: force
 // kernel of 1M particles in 2D 95.9 -> 88.3 us, of 4M in 3D blobs 1383 ->
 // 1187 us.)
-// Returns the number of cells staged (the same in every thread): as many of
-// the first ones as fit, 0 when not even one does; ncell <= kCells is the
+// Returns the number of cells staged to their end (the same in every thread):
+// as many of the first ones as fit; 0 when not even one does, with its first
+// kCap members (after the skipped ones) staged.  ncell <= kCells is the
 // caller's.
 template <int D, int V>
 __device__ __forceinline__ int stage_cells(const ForceArgs<D>& A, const ForceParams& P,
-                                           const uint32_t* __restrict__ cs, TileSmem<D, V>& sm, int off, int ncell) {
+                                           const uint32_t* __restrict__ cs, TileSmem<D, V>& sm, int off, int ncell,
+                                           int skip) {
     constexpr int R = TileRows<D>::R;
     constexpr int kT = TileCfg<D, V>::kTargets;
     constexpr int kPer = (TileCfg<D, V>::kCells + kT - 1) / kT;
@@ -271,6 +273,10 @@ __device__ __forceinline__ int stage_cells(const ForceArgs<D>& A, const ForcePar
             const int c = (rz * nx + ry) * nx + col;
             g0[i] = (int)__ldg(cs + c);
             len[i] = (int)__ldg(cs + c + 1) - g0[i];
+            if (e == 0) {
+                g0[i] += skip;
+                len[i] -= skip;
+            }
             sm.image[e] = P.wrap ? image : 0;
         }
         sum += len[i];
@@ -290,6 +296,7 @@ __device__ __forceinline__ int stage_cells(const ForceArgs<D>& A, const ForcePar
         before += w < warp ? x : 0;
         total += x;
     }
+    bool slice = false;
     if (total > TileCfg<D, V>::kCap) {  // block-uniform
         int fit = 0, end = before + inc - sum;
 #pragma unroll
@@ -304,7 +311,11 @@ __device__ __forceinline__ int stage_cells(const ForceArgs<D>& A, const ForcePar
         ncell = 0;
 #pragma unroll
         for (int w = 0; w < kT / 32; ++w) ncell += sm.wcol[w];
-        if (ncell == 0) return 0;
+        if (ncell == 0) {
+            slice = true;
+            ncell = 1;
+            if (tid == 0) len[0] = TileCfg<D, V>::kCap;
+        }
     }
     int run = before + inc - sum;
 #pragma unroll
@@ -333,13 +344,12 @@ __device__ __forceinline__ int stage_cells(const ForceArgs<D>& A, const ForcePar
     }
     copy_wait();
     __syncthreads();
-    return ncell;
+    return slice ? 0 : ncell;
 }
 
 // Main force kernel (nx >= 3): one thread per target; a block takes
 // kTargets consecutive targets and stages their windows
-// so that each target reads one contiguous run (or one per part, or, where a
-// cell does not fit, the same cells from global memory).  Neighbouring threads mostly share a cell, hence a
+// so that each target reads one contiguous run (or one per part).  Neighbouring threads mostly share a cell, hence a
 // window, so their candidate loads are broadcasts.  FP32 only: a target
 // whose neighbourhood holds a candidate that needs the FP64 decision is
 // deferred to its warp's closing pass (fixup_target), which recomputes it
@@ -483,10 +493,10 @@ __global__ void __launch_bounds__(TileCfg<D, V>::kTargets, TileCfg<D, V>::kMinBl
     const float4* const cand = sm.slots + TileSmem<D, V>::kLead;
     const float* Mrow = M + (valid ? Layout<D>::type(me) : 0) * ms;
     Acc acc = {0.f, 0.f, 0.f, 0, 0ull, 0ull, 0ull};
-    bool defer = false, direct = false;
+    bool defer = false;
     // 2D, the whole warp together (a lane without `mine` takes no part): the
     // target's staged cells lo .. up-1, its own cell being `own` (which may not
-    // be among them).  Only a target in the last column or row of a
+    // be among them, or not with the target's slice of it).  Only a target in the last column or row of a
     // periodic box meets candidates flagged for a target shift; its whole warp
     // then heeds the flags.
     auto evaluate2 = [&](bool mine, int lo, int up, int own, int ncell) {
@@ -513,7 +523,7 @@ __global__ void __launch_bounds__(TileCfg<D, V>::kTargets, TileCfg<D, V>::kMinBl
             j0 = sm.coff[lo];
             j1 = sm.coff[up];
             if ((unsigned)(own - lo) < (unsigned)(up - lo)) self = sm.coff[own] + (s - sm.cglob[own]);
-            if (DBG) acc.cand += j1 - j0 - (self >= 0 ? 1 : 0);
+            if (DBG) acc.cand += j1 - j0 - (self >= j0 && self < j1 ? 1 : 0);
         }
         // The lanes of a cell read the same candidates; the r-th cell of the
         // warp starts up to 7 before its window, at a staged index of r mod 8,
@@ -596,33 +606,24 @@ __global__ void __launch_bounds__(TileCfg<D, V>::kTargets, TileCfg<D, V>::kMinBl
     // window fits.  The parts follow in the window's order, hence the same
     // bits.  A staging may span segments: its columns are staged one by one
     // with their own rows, and a window never leaves its segment.  A cell that
-    // does not fit by itself sends the targets that need it to global memory.
+    // does not fit by itself comes in slices, the last of them with the cells
+    // after it.
     // (Whole windows per staging, a window that did not fit read from global
     // memory: 400k particles, 2D at 198 per cell, tile 1, 717 us a step, at
-    // 250 992; 3D at 50 per cell, tile 0, 825, tile 2 890.  In parts 589, 783,
-    // 560 and 587; whole columns per part 621, 820, 608 and 620.)
+    // 250 992; 3D at 50 per cell, tile 0, 825, tile 2 890; 16 and 128 worlds
+    // clustered for 620 steps 1018 and 9237.  In parts 602, 784, 560, 570, 892
+    // and 8345; whole columns per part 621, 820, 608 and 620.)
     constexpr int kCols = TileSmem<D, V>::kCols;
-    for (int a = 0; a < R * ncol;) {
+    for (int a = 0, skip = 0; a < R * ncol;) {
         const int c = a / R, off = a - c * R, hi = min(c + kCols, ncol);
         fill_columns(c, hi);  // the previous staging no longer reads the columns
         __syncthreads();
-        const int m = stage_cells<D, V>(A, P, cs, sm, off, R * (hi - c) - off);
+        const int m = stage_cells<D, V>(A, P, cs, sm, off, R * (hi - c) - off, skip);
         const int w = R * kwin - a;  // the window's first cell in this staging
-        const int lo = max(w, 0);
-        if (m > 0) {
-            const int up = min(w + 3 * R, m);
-            evaluate(valid && lo < up, lo, up, w + R + R / 2, m);
-            a += m;
-        } else {
-            direct |= valid && w <= 0 && w + 3 * R > 0;  // computed after the loop, off the hot path
-            ++a;
-        }
-    }
-    if (direct) {
-        // A cell did not fit in shared memory: the same sum from global
-        // memory, in place of the parts summed so far.
-        acc = {0.f, 0.f, 0.f, 0, 0ull, 0ull, 0ull};
-        defer = direct_stencil<D, DBG>(A, P, cs, Mrow, s, px, py, pz, cx, cy, cz, acc);
+        const int staged = max(m, 1), lo = max(w, 0), up = min(w + 3 * R, staged);
+        evaluate(valid && lo < up, lo, up, w + R + R / 2, staged);
+        a += m;
+        skip = m > 0 ? 0 : skip + TileCfg<D, V>::kCap;
     }
     const bool done = valid && !defer;
     uint32_t newcell = 0;
