@@ -438,7 +438,8 @@ int plg_batch_step_stats(plg_batch* batch, int64_t* deferred);
  * 2176, 1 = 64 / 944 (sparse worlds), 2 = 128 / 1776 (large worlds).
  * All give the same bits.  The worlds for which no variant was set or tuned
  * are on variant 0, or on 1 while the whole batch consists of crowded 2D worlds
- * (plg_set_tile).  After plg_batch_set_tile or plg_batch_autotune new worlds
+ * (plg_set_tile) and for 2D worlds of 100,000 particles or more at 100 per cell
+ * or more.  After plg_batch_set_tile or plg_batch_autotune new worlds
  * join with its variant.  Each world
  * of a batch has its own variant; a step launches the force kernel once per
  * variant in use.  The cell size is not a tuning choice: it is rmax (the

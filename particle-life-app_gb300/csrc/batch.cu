@@ -284,19 +284,26 @@ int check_desc(plg_batch* b, const plg_world_desc& d) {
 
 // The tile variant of the worlds for which none was set or tuned, whenever
 // the membership changes: the dense one where the whole batch is crowded, so
-// that it never opens a second force launch.  That costs every step more than
-// the dense tile gives the crowded worlds of a mixed batch, but for the largest
-// (a fork and join, and no chaining of steps).  15 worlds of 3,000 to 10,000
-// particles and one of n at d per cell, dense tile for that one against one
-// launch: n 432, d 48: 34.7 / 33.5 us a step; 5,000, 62: 51.4 / 47.2; 50,000,
-// 80: 80.7 / 78.6; 200,000, 125: 232 / 246; 20,000 in blobs, 62: 332 / 307.
+// that it opens no second force launch.  That costs every step more (a fork
+// and join, and no chaining of steps) than the dense tile gives the crowded
+// worlds of a mixed batch, unless they are large and dense.  15 worlds of 3,000
+// to 10,000 particles and one of n at d per cell, the dense tile for that one
+// against one launch: n 432, d 48: 33.4 / 33.0 us a step; 5,000, 62: 49.5 /
+// 46.5; 50,000, 80: 79.4 / 77.3; 50,000, 125: 118 / 120; 20,000 in blobs, 62:
+// 319 / 306; 200,000, 80: 150 / 151; 200,000, 125: 227 / 244; 200,000, 208:
+// 400 / 416.
+constexpr int64_t kApartParticles = 100000, kApartCell = 100;
+bool dense_apart(int dim, const WorldRec& w) {
+    return dim == 2 && w.n >= kApartParticles && w.n >= kApartCell * w.ncells;
+}
+
 void assign_variants(plg_batch* b) {
     if (!b->variant_auto) return;
     bool crowded = true;
     for (const WorldRec& w : b->worlds)
         if (!w.dead && w.n > 0) crowded &= w.variant_set ? w.variant == 1 : crowded_world(b->dim, w.n, w.ncells);
     for (WorldRec& w : b->worlds)
-        if (!w.variant_set) w.variant = crowded ? 1 : b->variant;
+        if (!w.variant_set) w.variant = crowded || (!w.dead && dense_apart(b->dim, w)) ? 1 : b->variant;
 }
 
 // The force kernel's tile tables: for each variant v, the first tile of

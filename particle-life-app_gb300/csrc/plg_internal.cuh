@@ -408,8 +408,8 @@ int tile_targets(int dim, int variant);
 
 // A 2D world with this many particles per cell on average takes the dense
 // tile (variant 1) until a variant is set or tuned: 400k particles, a step,
-// variant 0 against 1: 119 per cell 375 / 337 us, 198 per cell 635 / 589, 250
-// 810 / 783, 309 equal; a clustered world is only denser where its particles
+// variant 0 against 1: 119 per cell 371 / 341 us, 198 per cell 633 / 602, 250
+// 805 / 784, 309 1020 / 998; a clustered world is only denser where its particles
 // are.  (In a batch: assign_variants.)
 constexpr int64_t kCrowdedCell2D = 48;
 inline bool crowded_world(int dim, int64_t n, int64_t ncells) { return dim == 2 && n >= kCrowdedCell2D * ncells; }

@@ -1,6 +1,6 @@
-"""Tile variants that a batch gives its worlds: crowded 2D worlds never open a
-force launch of their own, whatever joins or leaves, and a variant set for a
-world stays."""
+"""Tile variants that a batch gives its worlds: crowded 2D worlds open no force
+launch of their own unless they are large and dense, whatever joins or leaves,
+and a variant set for a world stays."""
 import numpy as np
 import pytest
 
@@ -38,6 +38,19 @@ def test_one_launch_whatever_joins(gpu):
         assert tiles() == [2, 1]
         b.update(add=[dense])  # the set variant stays, and the batch is not on the dense tile throughout
         assert tiles() == [2, 0, 0]
+    finally:
+        b.close()
+
+
+@pytest.mark.parametrize("n,nx,tile", [(100_000, 31, 1), (99_999, 31, 0), (102_400, 32, 1), (102_399, 32, 0)])
+def test_large_dense_worlds_have_their_launch(gpu, n, nx, tile):
+    from plgpu.batch import GpuBatch
+
+    b = GpuBatch(2, 110_000, 4, 10_000)
+    try:
+        b.update(add=[_desc(3000, 50, 1), _desc(n, nx, 6)])
+        assert [b.world_tile(i) for i in b.world_ids()] == [0, tile]
+        b.step(2)
     finally:
         b.close()
 
