@@ -142,8 +142,9 @@ __global__ void __launch_bounds__(kThreads) k_force_general(const __grid_constan
 // 2D: tiles of 128 targets throughout (256 at 4 blocks per SM lose 2% at 6
 // particles per cell and 30% at 3 and below, where their windows need more
 // than the 256 stencil cells).  Variant 0: 8 blocks at 64 registers.  Variant
-// 1: 2048 candidates at 6 blocks for crowded cells (400k particles, 119 per
-// cell: 330 us against 498, 60 per cell: 169 against 172).  Variant 2: 7
+// 1: 2048 candidates at 6 blocks for crowded cells (400k particles, 123 per
+// cell: 336 us against 367, 250 per cell: 765 against 794, 61 per cell: 169
+// against 167).  Variant 2: 7
 // blocks with more registers and candidates, for worlds of about one wave.
 // 3D: 71 staged columns of 9 cells in variants 0 and 2, so that the sparse
 // tails of a blob world stage in one or two rounds.  Variant 0: 4 blocks of
@@ -153,10 +154,10 @@ __global__ void __launch_bounds__(kThreads) k_force_general(const __grid_constan
 // which did not fit beside 832 candidates, 9 ran with too few registers: 250k
 // uniform 95 us, now 90; 10 blocks of 808 candidates 96).  Variant 2:
 // 5 blocks of 128 targets with 1776 candidates, as much shared memory as five
-// blocks have, for large worlds (4M in blobs 1066 us against variant 0's 1148;
-// with 448 cells it took 1108, with 832 cells and 1600 candidates 1124; 1M at
-// 2.5 per cell 135 us against 147, 163 with 448 cells; six blocks of 1216
-// candidates 165).
+// blocks have, for large worlds (4M in blobs 1045 us against variant 0's 1135;
+// 1M at 2.4 per cell 127 us against 141.  With 448 cells 4% longer in blobs and
+// 21% at 2.4 per cell, with 832 cells and 1600 candidates 5% in blobs, with six
+// blocks of 1216 candidates 22% at 2.4 per cell).
 template <int D, int V>
 struct TileCfg;
 template <>

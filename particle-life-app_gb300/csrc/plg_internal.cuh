@@ -408,8 +408,8 @@ int tile_targets(int dim, int variant);
 
 // A 2D world with this many particles per cell on average takes the dense
 // tile (variant 1) until a variant is set or tuned: 400k particles, a step,
-// variant 0 against 1: 119 per cell 371 / 341 us, 198 per cell 633 / 602, 250
-// 805 / 784, 309 1020 / 998; a clustered world is only denser where its particles
+// variant 0 against 1: 48 per cell 151 / 153 us, 61 181 / 182, 123 384 / 347,
+// 198 633 / 602, 250 805 / 782, 309 1020 / 998; a clustered world is only denser where its particles
 // are.  (In a batch: assign_variants.)
 constexpr int64_t kCrowdedCell2D = 48;
 inline bool crowded_world(int dim, int64_t n, int64_t ncells) { return dim == 2 && n >= kCrowdedCell2D * ncells; }
@@ -417,11 +417,11 @@ inline bool crowded_world(int dim, int64_t n, int64_t ncells) { return dim == 2 
 // A 3D world below this many particles per cell on average is better off with
 // five blocks per SM (variant 2) than with variant 0's longer staging of
 // denser cells, once it fills the machine (kFullWorld3D): 1M particles, force
-// kernel, variant 0 -> 2: 2.4 per cell 147 -> 135 us, 6.0 per cell 188 -> 173,
-// 10.3 per cell 268 -> 255, 12.6 per cell 316 -> 320, 27.8 per cell 718 -> 812;
-// 4M in blobs, 0.3 per cell, 1148 -> 1066.  A world that clusters further
-// keeps the gain (the mean does not see it): 1M in blobs of 0.03 with 40
-// neighbours 308 -> 288.
+// kernel, variant 0 -> 2: 2.4 per cell 141 -> 127 us, 6.0 per cell 185 -> 172,
+// 10.3 per cell 261 -> 246, 12.6 per cell 306 -> 290, 27.8 per cell 603 -> 619;
+// 4M in blobs, 0.3 per cell, 1135 -> 1045.  (The line was drawn when windows
+// beyond variant 2's staging cost more: 12.6 per cell 316 -> 320, 27.8 718 ->
+// 812.)  A world that clusters further keeps the gain (the mean does not see it).
 constexpr int64_t kDenseCell3D = 11;
 inline bool open_world(int dim, int64_t n, int64_t ncells) { return dim == 3 && n < kDenseCell3D * ncells; }
 

@@ -313,13 +313,14 @@ void compute_force_params(plg_ctx* c) {
 Grid grid_of(plg_ctx* c) { return c->fp.g; }
 
 // 2D worlds below this many particles default to tile variant 2: they fill
-// at most two waves of blocks, and its extra registers count for more than
-// variant 0's eighth block.
+// at most two waves of blocks, and its extra registers count for as much as
+// variant 0's eighth block (force kernel at 6 per cell, variant 0 -> 2: 100k
+// 18.4 -> 18.4 us, 200k 24.8 -> 25.0, 290k 30.6 -> 31.2, 400k 37.1 -> 38.1).
 constexpr int64_t kSmallWorld2D = 300000;
 // 3D worlds of this many particles run more than two waves of blocks, where
-// variant 2's fifth block per SM counts (250k particles at 2.4 per cell 49 ->
-// 44 us, at 9.3 per cell 82 -> 82); at one wave it only lengthens the wave
-// (120k at 2.6 per cell: 30 -> 36 us).
+// variant 2's fifth block per SM counts (250k particles at 2.4 per cell 50 ->
+// 45 us, at 9.3 per cell 80 -> 75); at one wave it does not (120k at 2.6 per
+// cell 30 -> 31 us, at 8.7 47 -> 48).
 constexpr int64_t kFullWorld3D = 200000;
 
 // The tile variant a step uses: the one set or tuned, else by size.
